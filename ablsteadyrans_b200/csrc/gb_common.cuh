@@ -48,6 +48,48 @@ __host__ __device__ __forceinline__ int lateral_image(int i, int n_valid, int n,
     return (i < 0) ? i + n : i - n;
 }
 
+// --------------------------------------------------- division by extents ---
+
+//! n / d for 0 <= n < 2^31 and a divisor known at the launch, as one multiply
+//! and one shift: with s = ceil(log2 d) and m = floor(2^(31 + s) / d) + 1,
+//! n / d = (n m) >> (31 + s) exactly (the excess of m is at most d / 2^(31 + s)
+//! of the quotient, below the 1 / d that separates quotients for n < 2^31). A
+//! 64-bit division, which the linear kernels used to take twice a point to
+//! find their cell, is a routine of some hundred instructions.
+struct FastDiv {
+    uint32_t m{0};
+    int sh{0};
+    int d{1};
+    FastDiv() = default;
+    __host__ explicit FastDiv(int div) : d(div)
+    {
+        int s = 0;
+        while ((int64_t(1) << s) < div) { ++s; }
+        sh = 31 + s;
+        m = static_cast<uint32_t>((uint64_t(1) << sh) / static_cast<uint64_t>(div) + 1);
+    }
+    __host__ __device__ __forceinline__ int quot(int n) const
+    {
+        return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * m) >> sh);
+    }
+};
+
+//! The padded offset of valid cell n (i fastest) of a grid.
+struct CellMap {
+    FastDiv nx, ny;
+    int o0, sy, sz, n;
+    __host__ explicit CellMap(const gb_grid& g)
+        : nx(g.nx), ny(g.ny), o0(static_cast<int>(at(g, 0, 0, 0))), sy(static_cast<int>(g.sy)),
+          sz(static_cast<int>(g.sz)), n(g.nx * g.ny * g.nz)
+    {
+    }
+    __device__ __forceinline__ int offset(int c) const
+    {
+        const int r = nx.quot(c), k = ny.quot(r);
+        return o0 + (c - r * nx.d) + (r - k * ny.d) * sy + k * sz;
+    }
+};
+
 // ---------------------------------------------------------- reductions ---
 
 __device__ __forceinline__ double warp_max(double v)

@@ -257,8 +257,8 @@ __device__ __forceinline__ void resolve_neighbours(int i, int n, int periodic, i
 //! indices and mirror signs resolved once, a neighbour's value the product of
 //! its directions' signs (+-1, exact) times one load at the resolved point,
 //! ldc's value (the composition of per-direction reflections and shifts).
-template <typename T>
-__device__ __forceinline__ T adotx_cell(const gb_grid& g, const PBC& b, int i, int j, int k, const T* x,
+template <typename T, typename TX>
+__device__ __forceinline__ T adotx_cell(const gb_grid& g, const PBC& b, int i, int j, int k, const TX* x,
                                         const T* __restrict__ axa, const T* __restrict__ aya,
                                         const T* __restrict__ aza, const T* __restrict__ Jc, const MeshRatios<T>& m)
 {
@@ -274,7 +274,7 @@ __device__ __forceinline__ T adotx_cell(const gb_grid& g, const PBC& b, int i, i
     const int cz[3] = {(km + ng) * sz, (k + ng) * sz, (kp + ng) * sz};
     const int sx3[3] = {sim, 1, sip}, sy3[3] = {sjm, 1, sjp}, sz3[3] = {skm, 1, skp};
     auto X = [&](int di, int dj, int dk) {
-        const T v = x[cx[di + 1] + cy[dj + 1] + cz[dk + 1]];
+        const T v = static_cast<T>(x[cx[di + 1] + cy[dj + 1] + cz[dk + 1]]);
         return (sx3[di + 1] * sy3[dj + 1] * sz3[dk + 1] < 0) ? -v : v;
     };
     const int64_t o = at(g, i, j, k);

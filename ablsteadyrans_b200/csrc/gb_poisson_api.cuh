@@ -64,6 +64,7 @@ struct gb_poisson {
     double* t{nullptr};
     int dot_blocks{0};
     double* d_partial{nullptr};
+    unsigned* d_ticket{nullptr};  // the reductions' block counter (zero between launches)
     double* d_dots{nullptr};
     double* d_coef{nullptr};
     double* h_dots{nullptr};

@@ -457,3 +457,42 @@ def test_gpu_tma_tiles_solve_matches_oracle(ctx):
     y_ref = oracle.poisson_apply(g, bc, ax, ay, az, J, z, got.copy())
     v = g.valid(0)
     assert np.abs(y_ref[v] - rhs[v]).max() <= 1e-9 * np.abs(rhs[v]).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [(24, 20, 9, False, False, 0), (31, 17, 12, True, False, 0), (112, 80, 40, False, True, 0),
+                                  (112, 80, 40, True, True, 0), (48, 40, 21, False, False, 1)])
+@pytest.mark.parametrize("restart", [3, 50])
+def test_gpu_krylov_passes_meet_the_oracles_operator(ctx, case, restart):
+    """The Gram-Schmidt passes (one cell a thread on the small grids, several
+    on the 112 x 80 x 40 one; up to eight vectors a chunk and more), with
+    restarts every 3 vectors and without: a solve to 1e-9 leaves a residual
+    of the oracle's operator of 1e-9 of the right-hand side (2-norm, up to
+    the rounding of the two operators), and the result reports that residual.
+    The right-hand side's ghosts hold values, which no sum may take."""
+    import ablsteadyrans_b200 as gb
+    nx, ny, nz, px, py, precision = case
+    g, z, J, ax, ay, az, _ = smooth_terrain_case(nx, ny, nz, px, py, hill=150.0)
+    bc = (PERIODIC if px else NEUMANN, PERIODIC if py else NEUMANN, NEUMANN,
+          PERIODIC if px else DIRICHLET, PERIODIC if py else NEUMANN, NEUMANN)
+    rng = np.random.default_rng(21)
+    v = g.valid(0)
+    rhs = g.np_zeros() + 1e3
+    rhs[v] = rng.standard_normal(rhs[v].shape)
+    dz, dJ, dax, day, daz = _gpu_case(g, z, J, ax, ay, az)
+    opts = gb.PoissonOptions.default(precision=precision, reltol=1e-9, restart=restart, max_iter=200)
+    ps = gb.PoissonSolver(ctx, g, dz, dJ, bc, opts)
+    ps.set_coeffs(dax, day, daz)
+    drhs, phi = to_dev(rhs), to_dev(g.np_zeros() + 7.0)
+    res = ps.solve(drhs, phi)
+    got, b = to_host(phi), to_host(drhs)[v]
+    ps.close()
+    y = oracle.poisson_apply(g, bc, ax, ay, az, J, z, got.copy())[v]
+    left = float(np.linalg.norm(b - y))
+    assert res.singular == int(px and py or DIRICHLET not in bc)
+    assert res.initial_residual == pytest.approx(float(np.linalg.norm(b)), rel=1e-12)
+    assert left <= 1.0001e-9 * res.initial_residual
+    assert res.final_residual == pytest.approx(left, rel=1e-3)
+    ghosts = np.ones(g.shape, dtype=bool)
+    ghosts[v] = False
+    assert not got[ghosts].any()
