@@ -133,7 +133,7 @@ template <typename T>
 __device__ __forceinline__ T flux_x_r(const gb_grid& g, const PBC& b, int i, int j, int k, const T* x,
                                       const MeshRatios<T>& m)
 {
-    const T dxinv = static_cast<T>(1.0 / g.dx), h = T(0.5);
+    const T dxinv = static_cast<T>(b.dxinv), h = T(0.5);
     const int64_t o = at(g, i, j, k);
 #define X(a, bb, c) ldc<T>(x, x, g, b, a, bb, c)
     T px_lo = (X(i, j, k) - X(i - 1, j, k)) * dxinv;
@@ -150,7 +150,7 @@ template <typename T>
 __device__ __forceinline__ T flux_y_r(const gb_grid& g, const PBC& b, int i, int j, int k, const T* x,
                                       const MeshRatios<T>& m)
 {
-    const T dyinv = static_cast<T>(1.0 / g.dy), h = T(0.5);
+    const T dyinv = static_cast<T>(b.dyinv), h = T(0.5);
     const int64_t o = at(g, i, j, k);
 #define X(a, bb, c) ldc<T>(x, x, g, b, a, bb, c)
     T py_lo = (X(i, j, k) - X(i, j - 1, k)) * dyinv;
@@ -167,7 +167,7 @@ template <typename T>
 __device__ __forceinline__ T flux_z_r(const gb_grid& g, const PBC& b, int i, int j, int k, const T* x,
                                       const MeshRatios<T>& m)
 {
-    const T dxinv = static_cast<T>(1.0 / g.dx), dyinv = static_cast<T>(1.0 / g.dy), h = T(0.5);
+    const T dxinv = static_cast<T>(b.dxinv), dyinv = static_cast<T>(b.dyinv), h = T(0.5);
     const int64_t o = at(g, i, j, k);
 #define X(a, bb, c) ldc<T>(x, x, g, b, a, bb, c)
     T pz_lo = X(i, j, k) - X(i, j, k - 1);
@@ -227,7 +227,7 @@ __global__ void k_fluxes(gb_grid g, PBC b, const double* __restrict__ phi, MeshR
 __device__ __forceinline__ double z_face_cross_r(const gb_grid& g, const PBC& b, int i, int j, int k,
                                                  const double* x, const MeshRatios<double>& m)
 {
-    const double dxinv = 1.0 / g.dx, dyinv = 1.0 / g.dy, h = 0.5;
+    const double dxinv = b.dxinv, dyinv = b.dyinv, h = 0.5;
     const int64_t o = at(g, i, j, k);
 #define X(a, bb, c) ldc<double>(x, x, g, b, a, bb, c)
     const double px_hi_md_lo = h * (X(i + 1, j, k) - X(i, j, k) + X(i + 1, j, k - 1) - X(i, j, k - 1)) * dxinv;
@@ -797,7 +797,11 @@ __global__ void __launch_bounds__(256) k_color_relax_fused(gb_grid g, PBC b, int
 //! the correction downwards through shared memory as each segment's affine
 //! map (the segmented z-line sweep's carries). A coarse level's few columns
 //! then keep many warps busy, where one thread per column walks every level.
-template <typename T, int L>
+//! ZERO: the first colour of a relaxation from a zero iterate. Its residual is
+//! the right-hand side (A 0 = 0), so r is the level's b, x is written and not
+//! read, and the block also zeroes the other colour's columns beside its own
+//! (the pair 2c, 2c + 1 of a row): no residual launch, no zeroing of x before.
+template <typename T, int L, bool ZERO>
 __global__ void __launch_bounds__(512) k_color_solve_seg(gb_grid g, int color, const T* __restrict__ r,
                                                          const T* __restrict__ TD, const T* __restrict__ TC,
                                                          const T* __restrict__ TU, T* __restrict__ x)
@@ -827,7 +831,17 @@ __global__ void __launch_bounds__(512) k_color_solve_seg(gb_grid g, int color, c
         D[q] = TD[o];
         IM[q] = TC[o];
         CP[q] = TU[o];
-        X0[q] = x[o];
+        X0[q] = ZERO ? T(0) : x[o];
+    }
+    if (ZERO) {
+        const int i2 = 2 * c + 1 - ((j + color) & 1);
+        if (c < half && i2 < g.nx) {
+            const int64_t o2 = at(g, i2, j, 0);
+#pragma unroll
+            for (int q = 0; q < L; ++q) {
+                if (k0 + q < nz) { x[o2 + static_cast<int64_t>(k0 + q) * g.sz] = T(0); }
+            }
+        }
     }
     {
         T al = T(0), be = T(1);
@@ -1041,9 +1055,44 @@ __device__ __forceinline__ void prolong_cell(const gb_grid& gc, const PBC& bcb, 
     xf[at(gf, i, j, k)] += v * T(0.0625);
 }
 
+//! Coarse right-hand side straight from the fine iterate: a thread evaluates
+//! the residuals b - A x of fine cells (i, 2 J2) and (i, 2 J2 + 1) in turn, the
+//! lane beside it those of column i + 1, and the even lane adds the four as
+//! restrict_cell does. The fine residual never goes to memory and the level
+//! takes one launch where it took two. Two rows in turn (not unrolled) keep the
+//! operator's register count and occupancy.
+template <typename T>
+__global__ void __maxnreg__(72) k_residual_restrict(gb_grid gf, PBC b, const T* __restrict__ x, const T* __restrict__ bv,
+                                                    const T* __restrict__ AX, const T* __restrict__ AY,
+                                                    const T* __restrict__ AZ, const T* __restrict__ Jf, MeshRatios<T> m,
+                                                    gb_grid gc, const T* __restrict__ Jc, T* __restrict__ bc)
+{
+    pdl_entry();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int J2 = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    if (J2 >= gc.ny) { return; }               // whole warps: a row of threads is a warp
+    const int ii = min(i, gf.nx - 1);          // an in-range column for every lane of the exchange
+    T r0 = T(0), r1 = T(0);
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+        const int j = 2 * J2 + q;
+        const T r = bv[at(gf, ii, j, k)] - adotx_cell<T>(gf, b, ii, j, k, x, AX, AY, AZ, Jf, m);
+        if (q == 0) { r0 = r; } else { r1 = r; }
+    }
+    const T p0 = __shfl_down_sync(0xffffffffu, r0, 1), p1 = __shfl_down_sync(0xffffffffu, r1, 1);
+    if ((i & 1) || i >= gf.nx) { return; }     // nx is even: this level has a coarser one
+    const int j = 2 * J2;
+    const T s = (Jf[at(gf, i, j, k)] * r0 + Jf[at(gf, i + 1, j, k)] * p0)
+              + (Jf[at(gf, i, j + 1, k)] * r1 + Jf[at(gf, i + 1, j + 1, k)] * p1);
+    const int64_t oc = at(gc, i >> 1, J2, k);
+    bc[oc] = s / (T(4) * Jc[oc]);
+}
+
+//! The restriction of a residual in memory (the tiled operator's).
 template <typename T>
 __global__ void k_restrict(gb_grid gf, const T* __restrict__ Jf, const T* __restrict__ rf, gb_grid gc,
-                           const T* __restrict__ Jc, T* __restrict__ bc, T* __restrict__ xc)
+                           const T* __restrict__ Jc, T* __restrict__ bc)
 {
     pdl_entry();
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1051,9 +1100,6 @@ __global__ void k_restrict(gb_grid gf, const T* __restrict__ Jf, const T* __rest
     const int k = blockIdx.z;
     if (I >= gc.nx || J2 >= gc.ny) { return; }
     restrict_cell<T>(gf, Jf, rf, gc, Jc, bc, I, J2, k);
-    // the coarse correction starts from zero (its ghosts are never read: every
-    // kernel resolves a level's ghosts by index)
-    if (xc != nullptr) { xc[at(gc, I, J2, k)] = T(0); }
 }
 
 template <typename T>
@@ -1097,7 +1143,7 @@ __global__ void __launch_bounds__(256) k_coarse_relax(gb_grid g, PBC b, int nrel
     for (int n = threadIdx.x; n < plane; n += blockDim.x) {
         const int i = n % nx, j = (n / nx) % ny, k = n / (nx * ny);
         const int64_t o = at(g, i, j, k);
-        xs[n] = x[o];
+        xs[n] = T(0);  // the V-cycle's correction starts from zero
         sd[n] = TD[o];
         sm[n] = TC[o];
         sc[n] = TU[o];
@@ -1716,8 +1762,11 @@ void launch_tiles(gb_poisson* P, const gb_grid& g, const PBC& b, int color, cons
 //! Largest dynamic shared memory a relaxation kernel asks for.
 constexpr size_t kSmoothSmemMax = 200 * 1024;
 
+//! One zebra relaxation of level l. zero: the iterate is zero and x[l] need
+//! not hold it (the default column solves then skip the first colour's
+//! residual and write x whole; the other forms zero x first).
 template <typename T>
-void mg_smooth(gb_poisson* P, PoissonLevels<T>& L, int l)
+void mg_smooth(gb_poisson* P, PoissonLevels<T>& L, int l, bool zero)
 {
     gb_ctx* ctx = P->ctx;
     const bool pdl = ctx->tune[GB_TUNE_PDL] != 1;
@@ -1755,6 +1804,8 @@ void mg_smooth(gb_poisson* P, PoissonLevels<T>& L, int l)
     const int segW = (g.nz + segL - 1) / segL;
     // (GB_TUNE_MG_FUSED_RELAX 5: the segmented one-launch form on the levels
     // of at least 4096 columns only, the two launches below)
+    const bool own_solve = fknob < 2 && ctx->tune[GB_TUNE_MG_SOLVE] != 1 && (g.nz + 15) / 16 <= 16;
+    if (zero && !own_solve) { cudaMemsetAsync(L.x[l], 0, sizeof(T) * volume(g), ctx->stream); }
     const bool seg = (fknob == 4 || (fknob == 5 && g.nx * g.ny >= 4096)) && segW <= 16
                      && !(g.periodic_x && (g.nx & 1)) && !(g.periodic_y && (g.ny & 1));
     if (seg) {
@@ -1796,7 +1847,10 @@ void mg_smooth(gb_poisson* P, PoissonLevels<T>& L, int l)
     }
     for (int color = 0; color < 2; ++color) {
         Span span(ctx, GB_KERNEL_MG_SMOOTH);
-        if (use_tiles(P, g, L.x[l])) {
+        const bool first = zero && own_solve && color == 0;
+        if (first) {
+            --ctx->launches;  // no residual launch
+        } else if (use_tiles(P, g, L.x[l])) {
             launch_tiles<T, true>(P, g, b, color, L.x[l], L.AX[l], L.AY[l], L.AZ[l], L.J[l], L.ratios(l), L.bv[l],
                                   L.r[l]);
             --ctx->launches;  // counted with the solve below
@@ -1811,15 +1865,11 @@ void mg_smooth(gb_poisson* P, PoissonLevels<T>& L, int l)
         if (ctx->tune[GB_TUNE_MG_SOLVE] != 1 && sW <= 16) {
             // the segmented column solves (the default; GB_TUNE_MG_SOLVE = 1: one thread per column)
             const size_t sm = static_cast<size_t>(4) * sW * 32 * sizeof(T);
-            if (sL == 8) {
-                launch_pdl(pdl, k_color_solve_seg<T, 8>, dim3((half + 31) / 32, g.ny), dim3(32, sW), sm, ctx->stream, g,
-                           color, static_cast<const T*>(L.r[l]), static_cast<const T*>(L.TD[l]),
-                           static_cast<const T*>(L.TC[l]), static_cast<const T*>(L.TU[l]), L.x[l]);
-            } else {
-                launch_pdl(pdl, k_color_solve_seg<T, 16>, dim3((half + 31) / 32, g.ny), dim3(32, sW), sm, ctx->stream,
-                           g, color, static_cast<const T*>(L.r[l]), static_cast<const T*>(L.TD[l]),
-                           static_cast<const T*>(L.TC[l]), static_cast<const T*>(L.TU[l]), L.x[l]);
-            }
+            auto kern = sL == 8 ? (first ? k_color_solve_seg<T, 8, true> : k_color_solve_seg<T, 8, false>)
+                                : (first ? k_color_solve_seg<T, 16, true> : k_color_solve_seg<T, 16, false>);
+            launch_pdl(pdl, kern, dim3((half + 31) / 32, g.ny), dim3(32, sW), sm, ctx->stream, g, color,
+                       static_cast<const T*>(first ? L.bv[l] : L.r[l]), static_cast<const T*>(L.TD[l]),
+                       static_cast<const T*>(L.TC[l]), static_cast<const T*>(L.TU[l]), L.x[l]);
         } else if (staged) {
             launch_pdl(pdl, k_color_solve_staged<T>, sgrid, dim3(nthr), smem_staged, ctx->stream, g, color,
                        static_cast<const T*>(L.r[l]), static_cast<const T*>(L.TD[l]), static_cast<const T*>(L.TC[l]),
@@ -1861,21 +1911,27 @@ void build_line_tridiag(gb_poisson* P, PoissonLevels<T>& L)
     ctx->launches += 2;
 }
 
+//! The right-hand side of level l + 1 from the residual of level l.
 template <typename T>
-void mg_residual(gb_poisson* P, PoissonLevels<T>& L, int l)
+void mg_restrict(gb_poisson* P, PoissonLevels<T>& L, int l)
 {
     gb_ctx* ctx = P->ctx;
+    const bool pdl = ctx->tune[GB_TUNE_PDL] != 1;
     const gb_grid& g = L.g[l];
-    Span span(ctx, GB_KERNEL_POISSON_APPLY);
+    const gb_grid& gc = L.g[l + 1];
+    Span span(ctx, GB_KERNEL_MG_TRANSFER);
     if (use_tiles(P, g, L.x[l])) {
         launch_tiles<T, false>(P, g, L.b[l], -1, L.x[l], L.AX[l], L.AY[l], L.AZ[l], L.J[l], L.ratios(l), L.bv[l],
                                L.r[l]);
-        return;
+        launch_pdl(pdl, k_restrict<T>, cols_grid(gc, gc.nz), kColsBlock, 0, ctx->stream, g,
+                   static_cast<const T*>(L.J[l]), static_cast<const T*>(L.r[l]), gc, static_cast<const T*>(L.J[l + 1]),
+                   L.bv[l + 1]);
+    } else {
+        launch_pdl(pdl, k_residual_restrict<T>, dim3((g.nx + 31) / 32, (gc.ny + 3) / 4, g.nz), kColsBlock, 0,
+                   ctx->stream, g, L.b[l], static_cast<const T*>(L.x[l]), static_cast<const T*>(L.bv[l]),
+                   static_cast<const T*>(L.AX[l]), static_cast<const T*>(L.AY[l]), static_cast<const T*>(L.AZ[l]),
+                   static_cast<const T*>(L.J[l]), L.ratios(l), gc, static_cast<const T*>(L.J[l + 1]), L.bv[l + 1]);
     }
-    launch_pdl(ctx->tune[GB_TUNE_PDL] != 1, k_apply<T, T>, cols_grid(g, g.nz), kColsBlock, 0, ctx->stream, g, L.b[l],
-               static_cast<const T*>(L.x[l]), static_cast<const T*>(L.AX[l]), static_cast<const T*>(L.AY[l]),
-               static_cast<const T*>(L.AZ[l]), static_cast<const T*>(L.J[l]), L.ratios(l),
-               static_cast<const T*>(L.bv[l]), L.r[l], static_cast<T*>(nullptr));
     ++ctx->launches;
 }
 
@@ -1975,6 +2031,7 @@ bool mg_tail(gb_poisson* P, PoissonLevels<T>& L, int l)
         v.TU = L.TU[m];
     }
     const int pl = (L.g[l].nz + 31) / 32;
+    cudaMemsetAsync(L.x[l], 0, sizeof(T) * volume(L.g[l]), ctx->stream);
     Span span(ctx, GB_KERNEL_MG_SMOOTH);
     cudaError_t e = cudaErrorInvalidValue;
     switch (pl) {
@@ -2029,20 +2086,14 @@ void vcycle(gb_poisson* P, PoissonLevels<T>& L, int l)
             ++ctx->launches;
             return;
         }
-        for (int s = 0; s < P->opt.nu_coarse; ++s) { mg_smooth(P, L, l); }
+        for (int s = 0; s < P->opt.nu_coarse; ++s) { mg_smooth(P, L, l, s == 0); }
         return;
     }
-    for (int s = 0; s < P->opt.nu1; ++s) { mg_smooth(P, L, l); }
-    mg_residual(P, L, l);
     const gb_grid& gf = L.g[l];
     const gb_grid& gc = L.g[l + 1];
-    {
-        Span span(ctx, GB_KERNEL_MG_TRANSFER);
-        launch_pdl(pdl, k_restrict<T>, cols_grid(gc, gc.nz), kColsBlock, 0, ctx->stream, gf,
-                   static_cast<const T*>(L.J[l]), static_cast<const T*>(L.r[l]), gc, static_cast<const T*>(L.J[l + 1]),
-                   L.bv[l + 1], L.x[l + 1]);
-        ++ctx->launches;
-    }
+    if (P->opt.nu1 == 0) { cudaMemsetAsync(L.x[l], 0, sizeof(T) * volume(gf), ctx->stream); }
+    for (int s = 0; s < P->opt.nu1; ++s) { mg_smooth(P, L, l, s == 0); }
+    mg_restrict(P, L, l);
     vcycle(P, L, l + 1);
     {
         Span span(ctx, GB_KERNEL_MG_TRANSFER);
@@ -2050,7 +2101,7 @@ void vcycle(gb_poisson* P, PoissonLevels<T>& L, int l)
                    static_cast<const T*>(L.x[l + 1]), gf, L.x[l]);
         ++ctx->launches;
     }
-    for (int s = 0; s < P->opt.nu2; ++s) { mg_smooth(P, L, l); }
+    for (int s = 0; s < P->opt.nu2; ++s) { mg_smooth(P, L, l, false); }
 }
 
 //! A key of the tuning knobs that choose the V-cycle's kernels.
@@ -2123,12 +2174,9 @@ void run_vcycle(gb_poisson* P, PoissonLevels<T>& L, int ti)
 //! (FP64 or FP32) into its x[0].
 void vcycle_in_place(gb_poisson* P)
 {
-    gb_ctx* ctx = P->ctx;
     if (P->opt.precision == 1) {
-        cudaMemsetAsync(P->fl.x[0], 0, sizeof(float) * volume(P->g), ctx->stream);
         run_vcycle(P, P->fl, 1);
     } else {
-        cudaMemsetAsync(P->dl.x[0], 0, sizeof(double) * volume(P->g), ctx->stream);
         run_vcycle(P, P->dl, 0);
     }
 }
