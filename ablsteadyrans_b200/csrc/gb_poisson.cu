@@ -1029,6 +1029,141 @@ __global__ void __launch_bounds__(512) k_color_relax_seg(gb_grid g, PBC b, int c
     }
 }
 
+constexpr int kCellThreads = 512;
+
+//! One colour's relaxation in one launch, a cell a thread: a block takes
+//! C columns of the colour along a row, its threads evaluate
+//! r = b - A x of every cell (k_color_residual's operations) into shared memory
+//! with the columns' factors and x beside it, and the first threads run the
+//! segmented solves of k_color_solve_seg from there. Lateral neighbours are of
+//! the other colour and only this block writes its columns, so every read sees
+//! the values from before the update. Across the seam of a periodic direction
+//! of odd extent a column's neighbour has its own colour: there the launch
+//! writes another array (xo, the other colour copied beside), and a sweep's
+//! two colours go x -> r -> x.
+//! For the coarse levels, where a launch is latency: two launches a colour
+//! took 5.6 us whatever their few cells. Of 2, 4, 8 and 16 columns and 256,
+//! 384 and 512 threads, one cell for each of 512 threads was the fastest (FP64
+//! V-cycle of 32 x 32 x 48: 147 us with two launches, 132 so, 148 with 256
+//! threads, whose cells go in turn): 8 columns up to 64 levels, 4 up to 128.
+//! Taken where the level needs at most one such block an SM: V-cycles of
+//! 96 x 96 x 48 took 275 us with two launches, 237 so (144 blocks on its
+//! 48 x 48 level), 64 x 64 x 96 248 and 233, 30 x 30 x 18 (15 x 15 coarsest)
+//! 108 and 88. From two waves of blocks on the residual with one thread a cell
+//! over the whole chip is the better one (104 x 104 x 80: 318 us with its
+//! 52 x 52 level in two launches, 327 in one).
+template <typename T, int C>
+__global__ void __launch_bounds__(kCellThreads, 1)
+    k_color_relax_cells(gb_grid g, PBC b, int color, const T* x, T* xo, const T* __restrict__ bv, const T* __restrict__ AX,
+                        const T* __restrict__ AY, const T* __restrict__ AZ, const T* __restrict__ J, MeshRatios<T> m,
+                        const T* __restrict__ TD, const T* __restrict__ TC, const T* __restrict__ TU)
+{
+    constexpr int L = 8;
+    pdl_entry();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int nz = g.nz;
+    const int cap = C * nz;
+    T* sr = reinterpret_cast<T*>(smem_raw);  // [level][column]
+    T* sd = sr + cap;
+    T* si = sd + cap;
+    T* sc = si + cap;
+    T* sx = sc + cap;
+    const int W = (nz + L - 1) / L, cs = C * W;
+    T* carry = sx + cap;                     // [4][segment][column]
+    const int j = blockIdx.y;
+    const int tid = threadIdx.y * C + threadIdx.x;
+    {
+        const int odd = (j + color) & 1;
+        const int i = 2 * (blockIdx.x * C + threadIdx.x) + odd, i2 = i + 1 - 2 * odd, k = threadIdx.y;
+        if (x != xo && i2 < g.nx) { xo[at(g, i2, j, k)] = x[at(g, i2, j, k)]; }
+        if (i < g.nx) {
+            const int64_t o = at(g, i, j, k);
+            sd[tid] = TD[o];
+            si[tid] = TC[o];
+            sc[tid] = TU[o];
+            sx[tid] = x[o];
+            sr[tid] = bv[o] - adotx_cell<T>(g, b, i, j, k, x, AX, AY, AZ, J, m);
+        }
+    }
+    __syncthreads();
+    const int c = tid % C, w = tid / C;
+    const int i = 2 * (blockIdx.x * C + c) + ((j + color) & 1);
+    const bool act = w < W && i < g.nx;
+    const int k0 = w * L;
+    T R[L], D[L], IM[L], CP[L];
+    if (act) {
+#pragma unroll
+        for (int q = 0; q < L; ++q) {
+            const int e = min(k0 + q, nz - 1) * C + c;
+            R[q] = sr[e];
+            D[q] = sd[e];
+            IM[q] = si[e];
+            CP[q] = sc[e];
+        }
+        T al = T(0), be = T(1);
+#pragma unroll
+        for (int q = 0; q < L; ++q) {
+            const int k = k0 + q;
+            if (k < nz) {
+                if (k == 0) {
+                    al = R[q] * IM[q];
+                    be = T(0);
+                } else {
+                    al = (R[q] - D[q] * al) * IM[q];
+                    be = (-D[q] * be) * IM[q];
+                }
+            }
+        }
+        carry[tid] = al;
+        carry[cs + tid] = be;
+    }
+    __syncthreads();
+    if (act) {
+        T ep = T(0);
+#pragma unroll 4
+        for (int s = 0; s < w; ++s) { ep = carry[s * C + c] + carry[cs + s * C + c] * ep; }
+#pragma unroll
+        for (int q = 0; q < L; ++q) {
+            const int k = k0 + q;
+            if (k < nz) {
+                ep = (k == 0) ? R[q] * IM[q] : (R[q] - D[q] * ep) * IM[q];
+                R[q] = ep;
+            }
+        }
+        T ga = T(0), de = T(1);
+#pragma unroll
+        for (int q = L - 1; q >= 0; --q) {
+            const int k = k0 + q;
+            if (k < nz) {
+                if (k == nz - 1) {
+                    ga = R[q];
+                    de = T(0);
+                } else {
+                    ga = R[q] - CP[q] * ga;
+                    de = -CP[q] * de;
+                }
+            }
+        }
+        carry[2 * cs + tid] = ga;
+        carry[3 * cs + tid] = de;
+    }
+    __syncthreads();
+    if (act) {
+        T xk = T(0);
+#pragma unroll 4
+        for (int s = W - 1; s > w; --s) { xk = carry[2 * cs + s * C + c] + carry[3 * cs + s * C + c] * xk; }
+        const int64_t o0 = at(g, i, j, 0);
+#pragma unroll
+        for (int q = L - 1; q >= 0; --q) {
+            const int k = k0 + q;
+            if (k < nz) {
+                xk = (k == nz - 1) ? R[q] : R[q] - CP[q] * xk;
+                xo[o0 + static_cast<int64_t>(k) * g.sz] = sx[k * C + c] + xk;
+            }
+        }
+    }
+}
+
 //! Coarse right-hand side at coarse cell (I, J2, k): the J-weighted sum of
 //! the four fine residuals over 4 J_c (a coarse cell's flux balance is the sum
 //! of its fine cells').
@@ -1845,9 +1980,26 @@ void mg_smooth(gb_poisson* P, PoissonLevels<T>& L, int l, bool zero)
         }
         return;
     }
+    // one launch a colour where that takes at most one block an SM (see k_color_relax_cells)
+    const int ccols = g.nz <= kCellThreads / 8 ? 8 : 4;
+    const dim3 cgrid((half + ccols - 1) / ccols, g.ny);
+    const size_t csmem = (static_cast<size_t>(5) * ccols * g.nz + 4 * ccols * ((g.nz + 7) / 8)) * sizeof(T);
+    const bool cells = own_solve && ctx->tune[GB_TUNE_MG_STENCIL] != 2 && g.nz <= kCellThreads / 4
+                       && static_cast<int>(cgrid.x * cgrid.y) <= ctx->num_sms;
+    const bool split = (g.periodic_x && (g.nx & 1)) || (g.periodic_y && (g.ny & 1));
     for (int color = 0; color < 2; ++color) {
         Span span(ctx, GB_KERNEL_MG_SMOOTH);
         const bool first = zero && own_solve && color == 0;
+        if (cells && !first) {
+            launch_pdl(pdl, ccols == 8 ? k_color_relax_cells<T, 8> : k_color_relax_cells<T, 4>, cgrid,
+                       dim3(ccols, g.nz), csmem, ctx->stream, g, b, color, static_cast<const T*>(split && color == 1 ? L.r[l] : L.x[l]),
+                       split && color == 0 ? L.r[l] : L.x[l], static_cast<const T*>(L.bv[l]),
+                       static_cast<const T*>(L.AX[l]), static_cast<const T*>(L.AY[l]),
+                       static_cast<const T*>(L.AZ[l]), static_cast<const T*>(L.J[l]), L.ratios(l),
+                       static_cast<const T*>(L.TD[l]), static_cast<const T*>(L.TC[l]), static_cast<const T*>(L.TU[l]));
+            ++ctx->launches;
+            continue;
+        }
         if (first) {
             --ctx->launches;  // no residual launch
         } else if (use_tiles(P, g, L.x[l])) {
@@ -1869,7 +2021,8 @@ void mg_smooth(gb_poisson* P, PoissonLevels<T>& L, int l, bool zero)
                                 : (first ? k_color_solve_seg<T, 16, true> : k_color_solve_seg<T, 16, false>);
             launch_pdl(pdl, kern, dim3((half + 31) / 32, g.ny), dim3(32, sW), sm, ctx->stream, g, color,
                        static_cast<const T*>(first ? L.bv[l] : L.r[l]), static_cast<const T*>(L.TD[l]),
-                       static_cast<const T*>(L.TC[l]), static_cast<const T*>(L.TU[l]), L.x[l]);
+                       static_cast<const T*>(L.TC[l]), static_cast<const T*>(L.TU[l]),
+                       cells && split ? L.r[l] : L.x[l]);  // (only the first colour from zero comes here with cells)
         } else if (staged) {
             launch_pdl(pdl, k_color_solve_staged<T>, sgrid, dim3(nthr), smem_staged, ctx->stream, g, color,
                        static_cast<const T*>(L.r[l]), static_cast<const T*>(L.TD[l]), static_cast<const T*>(L.TC[l]),

@@ -496,3 +496,45 @@ def test_gpu_krylov_passes_meet_the_oracles_operator(ctx, case, restart):
     ghosts = np.ones(g.shape, dtype=bool)
     ghosts[v] = False
     assert not got[ghosts].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("case", [(15, 14, 18, True, False), (14, 15, 18, False, True), (13, 11, 70, True, True),
+                                  (96, 72, 7, False, False), (9, 7, 128, False, True), (33, 18, 2, True, False),
+                                  (40, 24, 129, False, False)])
+def test_gpu_one_launch_colours_give_the_two_launch_vcycle(ctx, case, precision):
+    """The one-launch colours (levels of at most one block an SM: odd and even
+    extents, a column's own colour across an odd periodic seam, columns of
+    two levels to more than half a block's threads, and of too many for it) run the
+    two launches' operations in their order. The two launches are what the
+    same hierarchy takes when its colours are relaxed by the sequential
+    column solves (GB_TUNE_MG_SOLVE 1), whose sums differ in the carries
+    across segments: equal to 1e-13 in FP64, 1e-5 in FP32; and the V-cycle of
+    the FP64 hierarchy equals the oracle's to 1e-12."""
+    import ablsteadyrans_b200 as gb
+    nx, ny, nz, px, py = case
+    g, z, J, ax, ay, az, _ = smooth_terrain_case(nx, ny, nz, px, py, hill=80.0)
+    bc = (PERIODIC if px else NEUMANN, PERIODIC if py else NEUMANN, NEUMANN,
+          PERIODIC if px else DIRICHLET, PERIODIC if py else DIRICHLET, DIRICHLET)
+    rng = np.random.default_rng(31)
+    v = g.valid(0)
+    r = g.np_zeros()
+    r[v] = rng.standard_normal(r[v].shape)
+    out = []
+    try:
+        for solve in (0, 1):
+            ctx.tune(gb.TUNE_MG_SOLVE, solve)
+            dz, dJ, dax, day, daz = _gpu_case(g, z, J, ax, ay, az)
+            ps = gb.PoissonSolver(ctx, g, dz, dJ, bc, gb.PoissonOptions.default(precision=precision))
+            ps.set_coeffs(dax, day, daz)
+            es = [to_host(ps.vcycle(to_dev(r))) for _ in range(2)]
+            assert np.array_equal(es[0], es[1])
+            out.append(es[0])
+            ps.close()
+    finally:
+        ctx.tune(gb.TUNE_MG_SOLVE, 0)
+    assert rel_err(out[0], out[1], v) < (1e-13 if precision == 0 else 1e-5)
+    if precision == 0:
+        mg = oracle.Multigrid(g, bc, z, J, ax, ay, az, max_levels=12, min_coarse=2, nu1=1, nu2=1, nu_coarse=8)
+        assert rel_err(out[0], mg.vcycle(r), v) < 1e-12
