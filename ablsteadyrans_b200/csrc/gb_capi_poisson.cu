@@ -32,8 +32,8 @@ gb_status gb::check_poisson_options(const gb_poisson_opts& o)
         gb::set_error("gust: invalid inputs: solver.poisson_max_iter must be >= 1");
         return GB_BAD_ARG;
     }
-    if (o.restart < 1 || o.restart > 200) {
-        gb::set_error("gust: invalid inputs: solver.poisson_restart must be >= 1 (and <= 200 here)");
+    if (o.restart < 1 || o.restart > gb::kMaxRestart) {
+        gb::set_error("gust: invalid inputs: solver.poisson_restart must be >= 1 (and <= %d here)", gb::kMaxRestart);
         return GB_BAD_ARG;
     }
     if (o.precision != 0 && o.precision != 1) {

@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 namespace gb {
@@ -1639,6 +1640,23 @@ __global__ void k_convert_all(T* __restrict__ dst, const double* __restrict__ sr
 // kBlock strided sums. A pass below keeps that order whatever it fuses, so the
 // iterates do not depend on how many launches a step takes.
 
+//! Krylov vectors as a kernel argument: at one stride (N = 0: those that a
+//! solver makes with itself, which most solves stop within), or up to N by
+//! address (they are made as a solve needs them). Addresses cost the passes: 1.5
+//! to 4 % of a whole projection (152 x 88 x 57, 17 steps), as a launch copies
+//! its parameters and every vector's address is a load.
+template <int N>
+struct Columns {
+    const double* p[N];
+    __device__ __forceinline__ const double* at(int q) const { return p[q]; }
+};
+template <>
+struct Columns<0> {
+    const double* base;
+    int64_t stride;
+    __device__ __forceinline__ const double* at(int q) const { return base + stride * q; }
+};
+
 constexpr int kDotWarps = kBlock / 32;
 constexpr int kDotChunk = 8;  // vectors whose sums a thread carries at once
 
@@ -1680,9 +1698,10 @@ __device__ __forceinline__ void finish_partials(const double* partial, int nq, d
 //! written) once for them, and an update and the products after it share the
 //! pass, so a step takes three passes (products; update and products; update
 //! and norm) in place of nine launches that read w once per vector.
-template <bool UPDATE, bool NORM>
-__global__ void __launch_bounds__(kBlock) k_gs_pass(CellMap cm, double* __restrict__ w, const double* __restrict__ V,
-                                                    int64_t vstride, int nq, const double* __restrict__ h,
+template <bool UPDATE, bool NORM, int N>
+__global__ void __launch_bounds__(kBlock) k_gs_pass(CellMap cm, double* __restrict__ w,
+                                                    const __grid_constant__ Columns<N> V, int nq,
+                                                    const double* __restrict__ h,
                                                     double* __restrict__ partial, double* __restrict__ out,
                                                     unsigned* __restrict__ ticket)
 {
@@ -1701,14 +1720,14 @@ __global__ void __launch_bounds__(kBlock) k_gs_pass(CellMap cm, double* __restri
             double v[kDotChunk];
             if (!NORM || UPDATE) {
 #pragma unroll
-                for (int e = 0; e < kDotChunk; ++e) { v[e] = (q0 + e < nq) ? V[vstride * (q0 + e) + o] : 0.0; }
+                for (int e = 0; e < kDotChunk; ++e) { v[e] = (q0 + e < nq) ? V.at(q0 + e)[o] : 0.0; }
             }
             if (UPDATE && q0 == 0) {
 #pragma unroll
                 for (int e = 0; e < kDotChunk; ++e) {
                     if (e < nq) { r -= h[e] * v[e]; }
                 }
-                for (int q = kDotChunk; q < nq; ++q) { r -= h[q] * V[vstride * q + o]; }
+                for (int q = kDotChunk; q < nq; ++q) { r -= h[q] * V.at(q)[o]; }
                 w[o] = r;
             }
             if (NORM) {
@@ -1761,15 +1780,18 @@ __global__ void __launch_bounds__(kBlock) k_dot_cells(CellMap cm, const double* 
     finish_partials(partial, 1, out, ticket);
 }
 
-//! phi += sum_q y[q] Z_q over the whole volume (Z's ghosts are zero).
-__global__ void __launch_bounds__(kBlock) k_add_combination(double* __restrict__ phi, const double* __restrict__ Z,
-                                                            int64_t vstride, int nq, const double* __restrict__ y, int n)
+//! phi += sum_q y[q] Z_q (valid cells).
+template <int N>
+__global__ void __launch_bounds__(kBlock) k_add_combination(CellMap cm, double* __restrict__ phi,
+                                                            const __grid_constant__ Columns<N> Z, int nq,
+                                                            const double* __restrict__ y)
 {
     pdl_entry();
-    const int o = blockIdx.x * kBlock + static_cast<int>(threadIdx.x);
-    if (o >= n) { return; }
+    const int c = blockIdx.x * kBlock + static_cast<int>(threadIdx.x);
+    if (c >= cm.n) { return; }
+    const int o = cm.offset(c);
     double s = phi[o];
-    for (int q = 0; q < nq; ++q) { s += y[q] * Z[vstride * q + o]; }
+    for (int q = 0; q < nq; ++q) { s += y[q] * Z.at(q)[o]; }
     phi[o] = s;
 }
 
@@ -1851,16 +1873,36 @@ void PoissonLevels<T>::release()
 
 }  // namespace gb
 
+void gb_poisson::release_chunks()
+{
+    if (chunks.empty()) { return; }
+    cudaStreamSynchronize(ctx->stream);
+    // the vectors in the chunks leave the lists; the others stay
+    const int64_t vol = (gb::volume(g) + 31) / 32 * 32;
+    auto ours = [&](const double* p) {
+        for (void* c : chunks) {
+            const double* b = static_cast<const double*>(c);
+            if (p >= b && p < b + vol * 2 * gb::kKrylovChunk) { return true; }
+        }
+        return false;
+    };
+    for (auto* list : {&Vc, &Zc, &spare}) {
+        list->erase(std::remove_if(list->begin(), list->end(), ours), list->end());
+    }
+    for (void* c : chunks) { cudaFree(c); }
+    chunks.clear();
+}
+
 gb_poisson::~gb_poisson()
 {
     for (int n = 0; n < 2; ++n) {
         if (vc_exec[n] != nullptr) { cudaGraphExecDestroy(vc_exec[n]); }
     }
     if (capture_stream != nullptr) { cudaStreamDestroy(capture_stream); }
+    release_chunks();
     for (void* p : owned) { cudaFree(p); }
     dl.release();
     fl.release();
-    if (h_dots) { cudaFreeHost(h_dots); }
     if (h_step) { cudaFreeHost(h_step); }
 }
 
@@ -2418,15 +2460,64 @@ void apply_to_vcycle(gb_poisson* P, double* zc, double* w)
     add_cross(P, zc, false, w);
 }
 
+//! The first n Krylov vectors of a list as a kernel argument.
+Columns<kMaxRestart> columns(const std::vector<double*>& c, int n)
+{
+    Columns<kMaxRestart> r;
+    for (int q = 0; q < n; ++q) { r.p[q] = c[q]; }
+    return r;
+}
+
+//! Whether the first n vectors of a list lie at one stride, and then as one.
+bool strided(const std::vector<double*>& c, int n, Columns<0>& r)
+{
+    r.base = c[0];
+    r.stride = n > 1 ? c[1] - c[0] : 0;
+    for (int q = 2; q < n; ++q) {
+        if (c[q] != c[0] + r.stride * q) { return false; }
+    }
+    return true;
+}
+
+//! n steps' Krylov vectors: Z of each, V of each and the one after.
+gb_status ensure_columns(gb_poisson* P, int n)
+{
+    const int64_t vol = (volume(P->g) + 31) / 32 * 32;
+    while (static_cast<int>(P->Zc.size()) < n || static_cast<int>(P->Vc.size()) < n + 1) {
+        if (P->spare.empty()) {
+            const int pairs = std::max(1, std::min(kKrylovChunk, P->opt.restart - static_cast<int>(P->Zc.size())));
+            void* p = nullptr;
+            if (cudaMalloc(&p, sizeof(double) * vol * 2 * pairs) != cudaSuccess) {
+                cudaGetLastError();
+                set_error("gust: PoissonSolver: cannot allocate the Krylov workspace");
+                return GB_OOM;
+            }
+            P->chunks.push_back(p);
+            for (int q = 0; q < 2 * pairs; ++q) { P->spare.push_back(static_cast<double*>(p) + vol * q); }
+        }
+        auto& to = P->Vc.size() <= P->Zc.size() ? P->Vc : P->Zc;
+        to.push_back(P->spare.back());
+        P->spare.pop_back();
+    }
+    return GB_OK;
+}
+
 //! One Gram-Schmidt pass (k_gs_pass) over w.
 template <bool UPDATE, bool NORM>
 void gs_pass(gb_poisson* P, int nq, const double* h, double* out)
 {
     gb_ctx* ctx = P->ctx;
     Span span(ctx, GB_KERNEL_VECTOR);
-    launch_pdl(ctx->tune[GB_TUNE_PDL] != 1, k_gs_pass<UPDATE, NORM>, dim3(P->dot_blocks), dim3(kBlock), 0, ctx->stream,
-               CellMap(P->g), P->w, static_cast<const double*>(P->V), P->vstride, nq, h, P->d_partial, out,
-               P->d_ticket);
+    const bool pdl = ctx->tune[GB_TUNE_PDL] != 1;
+    const dim3 grid(P->dot_blocks), block(kBlock);
+    Columns<0> v;
+    if (strided(P->Vc, nq, v)) {
+        launch_pdl(pdl, k_gs_pass<UPDATE, NORM, 0>, grid, block, 0, ctx->stream, CellMap(P->g), P->w, v, nq, h,
+                   P->d_partial, out, P->d_ticket);
+    } else {
+        launch_pdl(pdl, k_gs_pass<UPDATE, NORM, kMaxRestart>, grid, block, 0, ctx->stream, CellMap(P->g), P->w,
+                   columns(P->Vc, nq), nq, h, P->d_partial, out, P->d_ticket);
+    }
     ++ctx->launches;
 }
 
@@ -2470,10 +2561,70 @@ void basis_vector(gb_poisson* P, const double* w, const double* n2, double* vn)
 
 // ------------------------------------------------------------ creation ---
 
-gb_status poisson_build(gb_poisson* P)
+namespace {
+
+//! Hands out parts of one allocation: a first pass with no base adds up the
+//! bytes, a second deals them. A solver of six levels took some 130 cudaMalloc
+//! calls and as many cudaFree, milliseconds each way; now it takes three.
+struct Arena {
+    char* base{nullptr};
+    size_t used{0};
+    template <typename T>
+    T* take(int64_t n)
+    {
+        T* p = reinterpret_cast<T*>(base == nullptr ? nullptr : base + used);
+        used += (sizeof(T) * static_cast<size_t>(std::max<int64_t>(n, 1)) + 255) / 256 * 256;
+        return p;
+    }
+};
+
+//! One zeroed allocation for deal(Arena&), which is run twice.
+template <typename F>
+bool arena_alloc(cudaStream_t stream, std::vector<void*>& owned, F&& deal)
 {
-    gb_ctx* ctx = P->ctx;
-    // levels (FP64 geometry for every level, the FP32 copies when asked)
+    Arena a;
+    deal(a);
+    a.base = dalloc<char>(stream, owned, static_cast<int64_t>(a.used));
+    if (a.base == nullptr) { return false; }
+    a.used = 0;
+    deal(a);
+    return true;
+}
+
+//! The arrays of every level (level 0's geometry of the FP64 hierarchy is the
+//! caller's), with scratch areas of the coarse meshes' metrics for FP64.
+template <typename T>
+bool alloc_levels(gb_poisson* P, PoissonLevels<T>& L, const std::vector<gb_grid>& grids, double* (*metric)[3])
+{
+    return arena_alloc(P->ctx->stream, L.owned, [&](Arena& a) {
+        for (int l = 0; l < P->nlev; ++l) {
+            const int64_t vol = volume(grids[l]);
+            if (l > 0 || sizeof(T) == sizeof(float)) {
+                L.z[l] = a.take<T>(vol);
+                L.J[l] = a.take<T>(vol);
+            }
+            T** arrays[] = {L.AX, L.AY, L.AZ, L.x, L.bv, L.r, L.TD, L.TC, L.TU, L.RX, L.RY, L.HZ, L.SX, L.SY};
+            for (T** p : arrays) { p[l] = a.take<T>(vol); }
+            for (int n = 0; metric != nullptr && l > 0 && n < 3; ++n) { metric[l][n] = a.take<double>(vol); }
+        }
+    });
+}
+
+template <typename T>
+void borrow_levels(PoissonLevels<T>& L, const PoissonLevels<T>& from, int nlev)
+{
+    for (int l = 0; l < nlev; ++l) {
+        L.z[l] = from.z[l];
+        L.J[l] = from.J[l];
+        T** to[] = {L.AX, L.AY, L.AZ, L.x, L.bv, L.r, L.TD, L.TC, L.TU, L.RX, L.RY, L.HZ, L.SX, L.SY};
+        T* const* of[] = {from.AX, from.AY, from.AZ, from.x,  from.bv, from.r,  from.TD,
+                          from.TC, from.TU, from.RX, from.RY, from.HZ, from.SX, from.SY};
+        for (int n = 0; n < 14; ++n) { to[n][l] = of[n][l]; }
+    }
+}
+
+std::vector<gb_grid> level_grids(const gb_poisson* P)
+{
     std::vector<gb_grid> grids{P->g};
     while (static_cast<int>(grids.size()) < P->opt.max_levels) {
         const gb_grid& c = grids.back();
@@ -2481,132 +2632,118 @@ gb_status poisson_build(gb_poisson* P)
         if (!can) { break; }
         grids.push_back(coarse_grid(c));
     }
+    return grids;
+}
+
+}  // namespace
+
+bool poisson_can_lend(const gb_poisson* lender, const gb_poisson* P)
+{
+    return lender != nullptr && lender->ctx == P->ctx && lender->z_fine == P->z_fine && lender->J_fine == P->J_fine
+        && std::memcmp(&lender->g, &P->g, sizeof(gb_grid)) == 0
+        && lender->nlev == static_cast<int>(level_grids(P).size()) && lender->opt.precision >= P->opt.precision;
+}
+
+gb_status poisson_build(gb_poisson* P, gb_poisson* lender)
+{
+    gb_ctx* ctx = P->ctx;
+    // levels (FP64 geometry for every level, the FP32 copies when asked)
+    const std::vector<gb_grid> grids = level_grids(P);
     P->nlev = static_cast<int>(grids.size());
     auto& D = P->dl;
+    auto& F = P->fl;
     for (int l = 0; l < P->nlev; ++l) {
-        const gb_grid& g = grids[l];
-        D.g[l] = g;
-        D.b[l] = make_pbc(g, P->bc, P->bc[2] != PF_DIRICHLET);
-        const int64_t vol = volume(g);
-        if (l == 0) {
-            D.z[l] = const_cast<double*>(P->z_fine);
-            D.J[l] = const_cast<double*>(P->J_fine);
-        } else {
-            D.z[l] = dalloc<double>(ctx->stream, D.owned, vol);
-            D.J[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        }
-        D.AX[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.AY[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.AZ[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.x[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.bv[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.r[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.snap[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.TD[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.TC[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.TU[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.RX[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.RY[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.HZ[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.SX[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        D.SY[l] = dalloc<double>(ctx->stream, D.owned, vol);
-        if (!D.TD[l] || !D.TC[l] || !D.TU[l] || !D.RX[l] || !D.RY[l] || !D.HZ[l] || !D.SX[l] || !D.SY[l]) {
-            set_error("gust: PoissonSolver: cannot allocate the multigrid levels");
-            return GB_OOM;
-        }
-        if (!D.AX[l] || !D.AY[l] || !D.AZ[l] || !D.x[l] || !D.bv[l] || !D.r[l] || !D.snap[l] || (l > 0 && (!D.z[l] || !D.J[l]))) {
-            set_error("gust: PoissonSolver: cannot allocate the multigrid levels");
-            return GB_OOM;
-        }
-        if (l > 0) {
-            const gb_grid& gf = grids[l - 1];
-            const int64_t nz3 = static_cast<int64_t>(g.nx + 3) * (g.ny + 3) * (g.nz + 3);
-            k_coarse_z<<<nblocks(nz3), kBlock, 0, ctx->stream>>>(g, D.z[l], gf, D.z[l - 1]);
-            double* ax = dalloc<double>(ctx->stream, D.owned, vol);
-            double* ay = dalloc<double>(ctx->stream, D.owned, vol);
-            double* zcc = dalloc<double>(ctx->stream, D.owned, vol);
-            const int64_t nm = static_cast<int64_t>(g.nx + 3) * (g.ny + 3) * (g.nz + 2);
-            k_metrics<<<nblocks(nm), kBlock, 0, ctx->stream>>>(g, D.z[l], D.J[l], ax, ay, zcc);
-            ctx->launches += 2;
-        }
-        const int64_t nr = static_cast<int64_t>(g.nx + 1) * (g.ny + 1) * (g.nz + 1);
-        k_mesh_ratios<double><<<nblocks(nr), kBlock, 0, ctx->stream>>>(g, D.z[l], D.RX[l], D.RY[l], D.HZ[l], D.SX[l],
-                                                                       D.SY[l]);
-        ++ctx->launches;
+        D.g[l] = F.g[l] = grids[l];
+        D.b[l] = F.b[l] = make_pbc(grids[l], P->bc, P->bc[2] != PF_DIRICHLET);
     }
-    if (P->opt.precision == 1) {
-        auto& F = P->fl;
+    D.z[0] = const_cast<double*>(P->z_fine);
+    D.J[0] = const_cast<double*>(P->J_fine);
+    P->borrows = lender != nullptr;
+    if (lender != nullptr) {
+        borrow_levels(D, lender->dl, P->nlev);
+        if (P->opt.precision == 1) { borrow_levels(F, lender->fl, P->nlev); }
+    } else {
+        double* metric[kMaxLevels][3] = {};
+        if (!alloc_levels(P, D, grids, metric)) {
+            set_error("gust: PoissonSolver: cannot allocate the multigrid levels");
+            return GB_OOM;
+        }
         for (int l = 0; l < P->nlev; ++l) {
             const gb_grid& g = grids[l];
-            F.g[l] = g;
-            F.b[l] = D.b[l];
-            const int64_t vol = volume(g);
-            F.z[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.J[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.AX[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.AY[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.AZ[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.x[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.bv[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.r[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.snap[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.TD[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.TC[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.TU[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.RX[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.RY[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.HZ[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.SX[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            F.SY[l] = dalloc<float>(ctx->stream, F.owned, vol);
-            if (!F.TD[l] || !F.TC[l] || !F.TU[l] || !F.RX[l] || !F.RY[l] || !F.HZ[l] || !F.SX[l] || !F.SY[l]) {
-                set_error("gust: PoissonSolver: cannot allocate the FP32 multigrid levels");
-                return GB_OOM;
+            if (l > 0) {
+                const gb_grid& gf = grids[l - 1];
+                const int64_t nz3 = static_cast<int64_t>(g.nx + 3) * (g.ny + 3) * (g.nz + 3);
+                k_coarse_z<<<nblocks(nz3), kBlock, 0, ctx->stream>>>(g, D.z[l], gf, D.z[l - 1]);
+                const int64_t nm = static_cast<int64_t>(g.nx + 3) * (g.ny + 3) * (g.nz + 2);
+                k_metrics<<<nblocks(nm), kBlock, 0, ctx->stream>>>(g, D.z[l], D.J[l], metric[l][0], metric[l][1],
+                                                                   metric[l][2]);
+                ctx->launches += 2;
             }
             const int64_t nr = static_cast<int64_t>(g.nx + 1) * (g.ny + 1) * (g.nz + 1);
-            k_mesh_ratios<float><<<nblocks(nr), kBlock, 0, ctx->stream>>>(g, D.z[l], F.RX[l], F.RY[l], F.HZ[l],
-                                                                          F.SX[l], F.SY[l]);
+            k_mesh_ratios<double><<<nblocks(nr), kBlock, 0, ctx->stream>>>(g, D.z[l], D.RX[l], D.RY[l], D.HZ[l],
+                                                                           D.SX[l], D.SY[l]);
             ++ctx->launches;
-            if (!F.z[l] || !F.J[l] || !F.AX[l] || !F.AY[l] || !F.AZ[l] || !F.x[l] || !F.bv[l] || !F.r[l] || !F.snap[l]) {
+        }
+        if (P->opt.precision == 1) {
+            if (!alloc_levels(P, F, grids, nullptr)) {
                 set_error("gust: PoissonSolver: cannot allocate the FP32 multigrid levels");
                 return GB_OOM;
             }
-            k_convert_all<float><<<nblocks(vol), kBlock, 0, ctx->stream>>>(F.z[l], D.z[l], vol);
-            k_convert_all<float><<<nblocks(vol), kBlock, 0, ctx->stream>>>(F.J[l], D.J[l], vol);
-            ctx->launches += 2;
+            for (int l = 0; l < P->nlev; ++l) {
+                const gb_grid& g = grids[l];
+                const int64_t vol = volume(g);
+                const int64_t nr = static_cast<int64_t>(g.nx + 1) * (g.ny + 1) * (g.nz + 1);
+                k_mesh_ratios<float><<<nblocks(nr), kBlock, 0, ctx->stream>>>(g, D.z[l], F.RX[l], F.RY[l], F.HZ[l],
+                                                                              F.SX[l], F.SY[l]);
+                k_convert_all<float><<<nblocks(vol), kBlock, 0, ctx->stream>>>(F.z[l], D.z[l], vol);
+                k_convert_all<float><<<nblocks(vol), kBlock, 0, ctx->stream>>>(F.J[l], D.J[l], vol);
+                ctx->launches += 3;
+            }
         }
     }
-    // Krylov workspace
-    const int64_t vol = volume(P->g);
+    // Krylov workspace. The vectors of the first steps come with it: as many of
+    // the restart's as kKrylovBytes hold (8 at least); further ones when a solve
+    // gets that far. All of them (restart 50: 101 volumes) were 5.5 GB on a
+    // 256 x 256 x 96 grid whose solves take 8 to 20 steps.
+    constexpr int64_t kKrylovBytes = int64_t(512) << 20;
+    const int64_t vol = volume(P->g), vs = (vol + 31) / 32 * 32;
     const int m = P->opt.restart;
-    // the basis columns at a stride of whole 256-byte lines: every column's
-    // base is 16-byte aligned, as the TMA-staged operator tiles need
-    P->vstride = (vol + 31) / 32 * 32;
-    P->V = dalloc<double>(ctx->stream, P->owned, P->vstride * (m + 1));
-    P->Zv = dalloc<double>(ctx->stream, P->owned, P->vstride * m);
-    P->w = dalloc<double>(ctx->stream, P->owned, vol);
-    P->t = dalloc<double>(ctx->stream, P->owned, vol);
+    const int pairs = static_cast<int>(std::min<int64_t>(m, std::max<int64_t>(kKrylovChunk, kKrylovBytes / (16 * vs))));
     P->dot_blocks = std::min(4 * ctx->num_sms, nblocks(static_cast<int64_t>(P->g.nx) * P->g.ny * P->g.nz));
-    P->d_ticket = dalloc<unsigned>(ctx->stream, P->owned, 1);
-    P->d_partial = dalloc<double>(ctx->stream, P->owned, static_cast<int64_t>(P->dot_blocks) * (m + 2));
-    P->d_dots = dalloc<double>(ctx->stream, P->owned, m + 2);
-    P->d_coef = dalloc<double>(ctx->stream, P->owned, m + 2);
-    P->d_step = dalloc<double>(ctx->stream, P->owned, 3 * (m + 2));
-    P->d_err = dalloc<unsigned long long>(ctx->stream, P->owned, 1);
-    if (!P->V || !P->Zv || !P->w || !P->t || !P->d_partial || !P->d_dots || !P->d_coef || !P->d_err || !P->d_ticket) {
+    if (lender != nullptr) {
+        P->w = lender->w;
+        P->t = lender->t;
+        P->Vc = lender->Vc;
+        P->Zc = lender->Zc;
+        for (double* s : lender->spare) { P->spare.push_back(s); }
+    }
+    const bool ok = arena_alloc(ctx->stream, P->owned, [&](Arena& a) {
+        P->d_ticket = a.take<unsigned>(1);
+        P->d_partial = a.take<double>(static_cast<int64_t>(P->dot_blocks) * (m + 2));
+        P->d_dots = a.take<double>(m + 2);
+        P->d_coef = a.take<double>(m + 2);
+        P->d_step = a.take<double>(3 * (m + 2));
+        P->d_err = a.take<unsigned long long>(1);
+        if (lender == nullptr) {
+            P->w = a.take<double>(vol);
+            P->t = a.take<double>(vol);
+            P->Vc.clear();
+            P->Zc.clear();
+            for (int q = 0; q <= pairs; ++q) { P->Vc.push_back(a.take<double>(vs)); }
+            for (int q = 0; q < pairs; ++q) { P->Zc.push_back(a.take<double>(vs)); }
+        }
+    });
+    if (!ok) {
         set_error("gust: PoissonSolver: cannot allocate the Krylov workspace");
         return GB_OOM;
     }
-    if (cudaMallocHost(&P->h_step, sizeof(double) * 3 * (m + 2)) != cudaSuccess) {
+    if (cudaMallocHost(&P->h_step, sizeof(double) * 4 * (m + 2)) != cudaSuccess) {
         cudaGetLastError();
         P->h_step = nullptr;
         set_error("gust: PoissonSolver: out of pinned host memory");
         return GB_OOM;
     }
-    if (cudaMallocHost(&P->h_dots, sizeof(double) * (m + 2)) != cudaSuccess) {
-        cudaGetLastError();
-        set_error("gust: PoissonSolver: cannot allocate pinned host words");
-        return GB_OOM;
-    }
+    P->h_dots = P->h_step + 3 * (m + 2);
     return check_cuda("PoissonSolver");
 }
 
@@ -2802,14 +2939,16 @@ gb_status poisson_solve(gb_poisson* P, double* rhs, double* phi, gb_poisson_resu
             set_error("gust: the Poisson solve produced a non-finite residual");
             return GB_NONFINITE;
         }
-        basis_vector(P, r0, P->d_dots, P->V);
+        if ((st = ensure_columns(P, 1)) != GB_OK) { return st; }
+        basis_vector(P, r0, P->d_dots, P->Vc[0]);
         std::fill(s.begin(), s.end(), 0.0);
         std::fill(H.begin(), H.end(), 0.0);
         s[0] = beta;
         int jj = 0;
         for (; jj < m && it < P->opt.max_iter; ++jj) {
             ++it;
-            double* zj = P->Zv + P->vstride * jj;
+            if ((st = ensure_columns(P, jj + 1)) != GB_OK) { return st; }
+            double* zj = P->Zc[jj];
             vcycle_in_place(P);
             apply_to_vcycle(P, zj, P->w);
             // classical Gram-Schmidt, twice, and the norm of what is left: the
@@ -2824,7 +2963,7 @@ gb_status poisson_solve(gb_poisson* P, double* rhs, double* phi, gb_poisson_resu
             gs_pass<true, false>(P, jj + 1, d1, d2);
             gs_pass<true, true>(P, jj + 1, d2, dn);
             cudaMemcpyAsync(P->h_step, P->d_step, sizeof(double) * 3 * st3, cudaMemcpyDeviceToHost, ctx->stream);
-            basis_vector(P, P->w, dn, P->V + P->vstride * (jj + 1));
+            basis_vector(P, P->w, dn, P->Vc[jj + 1]);
             if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) { return check_cuda("poisson dot"); }
             for (int pass = 0; pass < 2; ++pass) {
                 for (int q = 0; q <= jj; ++q) { h[q] += P->h_step[pass * st3 + q]; }
@@ -2857,9 +2996,16 @@ gb_status poisson_solve(gb_poisson* P, double* rhs, double* phi, gb_poisson_resu
         }
         // (the host's copy of y is taken before the call returns: pageable memory)
         cudaMemcpyAsync(P->d_coef, y.data(), sizeof(double) * jj, cudaMemcpyHostToDevice, ctx->stream);
-        launch_pdl(ctx->tune[GB_TUNE_PDL] != 1, k_add_combination, dim3(nblocks(vol)), dim3(kBlock), 0, ctx->stream,
-                   phi, static_cast<const double*>(P->Zv), P->vstride, jj, static_cast<const double*>(P->d_coef),
-                   static_cast<int>(vol));
+        const CellMap cm(g);
+        const bool pdl = ctx->tune[GB_TUNE_PDL] != 1;
+        const double* yd = P->d_coef;
+        Columns<0> z;
+        if (strided(P->Zc, jj, z)) {
+            launch_pdl(pdl, k_add_combination<0>, dim3(nblocks(cm.n)), dim3(kBlock), 0, ctx->stream, cm, phi, z, jj, yd);
+        } else {
+            launch_pdl(pdl, k_add_combination<kMaxRestart>, dim3(nblocks(cm.n)), dim3(kBlock), 0, ctx->stream, cm, phi,
+                       columns(P->Zc, jj), jj, yd);
+        }
         ++ctx->launches;
         last = -1.0;
     }

@@ -8,6 +8,8 @@
 namespace gb {
 
 constexpr int kMaxLevels = 16;
+constexpr int kMaxRestart = 200;
+constexpr int kKrylovChunk = 8;
 
 //! The multigrid hierarchy in one arithmetic type.
 template <typename T>
@@ -22,7 +24,6 @@ struct PoissonLevels {
     T* x[kMaxLevels] = {};
     T* bv[kMaxLevels] = {};
     T* r[kMaxLevels] = {};
-    T* snap[kMaxLevels] = {};
     T* TD[kMaxLevels] = {};   // the smoother's line tridiagonal, per level
     T* TC[kMaxLevels] = {};
     T* TU[kMaxLevels] = {};
@@ -49,6 +50,7 @@ struct gb_poisson {
     gb::PoissonLevels<double> dl;  // FP64 hierarchy (geometry and coefficients of every level)
     gb::PoissonLevels<float> fl;   // FP32 copies (precision == 1)
     bool coeffs_set{false};
+    bool borrows{false};  // the level arrays are another solver's (poisson_build's lender)
     // FaceCoeffs::z_cross: d = beta_z - z_cross and a_z d per z-face (owned;
     // null: no split). The Krylov operator and the fluxes carry it, the
     // V-cycle (the preconditioner) does not.
@@ -56,9 +58,12 @@ struct gb_poisson {
     double* cross_ad{nullptr};
     double* cross_store[2]{nullptr, nullptr};
     // Krylov workspace
-    int64_t vstride{0};
-    double* V{nullptr};
-    double* Zv{nullptr};
+    // The basis and the preconditioned vectors, one padded volume each (their
+    // ghosts are never read): made as the steps of a solve need them, from
+    // `spare` volumes first (a lender's), then in chunks of kKrylovChunk pairs.
+    std::vector<double*> Vc, Zc;
+    std::vector<double*> spare;
+    std::vector<void*> chunks;
     unsigned long long* d_err{nullptr};    // set when a TMA tile wait gave up
     double* w{nullptr};
     double* t{nullptr};
@@ -82,6 +87,9 @@ struct gb_poisson {
     int vc_calls[2]{0, 0};
     uint64_t vc_tune_key[2]{0, 0};
     std::vector<void*> owned;
+    //! Gives the chunks of Krylov vectors back, after the work on the stream (a
+    //! later solve makes new ones).
+    void release_chunks();
     ~gb_poisson();
 };
 
@@ -89,7 +97,13 @@ namespace gb {
 
 //! The range checks of solver.poisson_* (messages name the keys).
 gb_status check_poisson_options(const gb_poisson_opts& o);
-gb_status poisson_build(gb_poisson* P);
+//! Builds the hierarchy and the Krylov workspace. lender: a solver of the same
+//! mesh on the same context, with the same levels and at least this precision
+//! (poisson_can_lend), whose level arrays and Krylov vectors this one uses while
+//! both live: whichever of the two sets its coefficients last is the one that
+//! may apply or solve. null: arrays of its own.
+gb_status poisson_build(gb_poisson* P, gb_poisson* lender = nullptr);
+bool poisson_can_lend(const gb_poisson* lender, const gb_poisson* P);
 gb_status poisson_set_coeffs(gb_poisson* P, const double* ax, const double* ay, const double* az, const double* bx,
                              const double* by, const double* bz);
 gb_status poisson_set_z_cross(gb_poisson* P, const double* az, const double* bz, const double* z_cross);

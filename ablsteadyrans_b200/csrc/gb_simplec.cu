@@ -3188,6 +3188,52 @@ void w_from_omega(gb_simplec* S, const double* u, const double* v, const double*
 
 }  // namespace
 
+//! The initializer's projection solver (its own boundary conditions and
+//! options). It works in the arrays of the stage's correction solver, which
+//! sets its coefficients before every solve, and takes its further Krylov
+//! vectors from the line systems' arrays, which every iteration fills anew; so
+//! the stage keeps it from call to call at no memory of note. A solver made and
+//! destroyed in every call spent 25 of the 30 ms of a 96 x 96 x 64 initial
+//! state in cudaMalloc and cudaFree.
+gb_status init_solver(gb_simplec* S, const int32_t* pbc, const gb_poisson_opts& po)
+{
+    gb_poisson* P = S->init_poisson;
+    if (P != nullptr && std::memcmp(P->bc, pbc, sizeof(P->bc)) == 0 && P->opt.max_levels == po.max_levels
+        && P->opt.min_coarse == po.min_coarse && P->opt.precision == po.precision && P->opt.restart == po.restart
+        && P->opt.nu1 == po.nu1 && P->opt.nu2 == po.nu2 && P->opt.nu_coarse == po.nu_coarse) {
+        P->opt = po;  // the tolerances and the iteration limit
+        return poisson_set_z_cross(P, nullptr, nullptr, nullptr);
+    }
+    if (P != nullptr) {
+        gb_poisson_destroy(P);
+        S->init_poisson = nullptr;
+    }
+    P = new (std::nothrow) gb_poisson;
+    if (P == nullptr) { return GB_OOM; }
+    P->ctx = S->ctx;
+    P->g = S->g;
+    std::memcpy(P->bc, pbc, sizeof(P->bc));
+    P->opt = po;
+    P->z_fine = S->z;
+    P->J_fine = S->mesh.detJ;
+    gb_poisson* lender = poisson_can_lend(S->poisson, P) ? S->poisson : nullptr;
+    if (lender != nullptr) {
+        const int64_t vol = volume(S->g);
+        double* lent[4] = {S->w.Am[0], S->w.Am[1], S->w.Am[2], S->w.At};
+        for (double* a : lent) {
+            for (int n = 0; n < GB_N_COEFS; ++n) { P->spare.push_back(a + vol * n); }
+        }
+    }
+    const gb_status st = poisson_build(P, lender);
+    if (st != GB_OK) {
+        cudaStreamSynchronize(S->ctx->stream);
+        delete P;
+        return st;
+    }
+    S->init_poisson = P;
+    return GB_OK;
+}
+
 gb_status simplec_initialize(gb_simplec* S, const gb_state& q, const gb_init_opts& o, gb_init_result* r)
 {
     gb_ctx* ctx = S->ctx;
@@ -3269,10 +3315,6 @@ gb_status simplec_initialize(gb_simplec* S, const gb_state& q, const gb_init_opt
     velocity_divergence(S, q.u, q.v, q.w, w.rhs);
     dsum(S, valid_box(g, CC), w.rhs, 0, 0);
     if (o.projection) {
-        if (S->init_poisson != nullptr) {
-            gb_poisson_destroy(S->init_poisson);
-            S->init_poisson = nullptr;
-        }
         // initializer_poisson_bc (Initializer.cpp:181-195): lambda = 0 on the
         // inflow and outflow faces, zero flux through the others
         int32_t pbc[6];
@@ -3284,7 +3326,7 @@ gb_status simplec_initialize(gb_simplec* S, const gb_state& q, const gb_init_opt
                                                                                      : GB_POISSON_NEUMANN);
         }
         gb_poisson_opts po = o.poisson;
-        gb_status st = gb_poisson_create(ctx, &g, pbc, S->z, S->mesh.detJ, &po, &S->init_poisson);
+        gb_status st = init_solver(S, pbc, po);
         if (st != GB_OK) { return st; }
         const bool unit = (o.alpha_h == 1 && o.alpha_v == 1);
         const double* beta[3] = {nullptr, nullptr, nullptr};
@@ -3332,9 +3374,13 @@ gb_status simplec_initialize(gb_simplec* S, const gb_state& q, const gb_init_opt
         }
         w_from_omega(S, q.u, q.v, w.om, q.w);
         velocity_divergence(S, q.u, q.v, q.w, w.rhs);
-        // the projection runs once per solve: its solver's memory goes back
-        gb_poisson_destroy(S->init_poisson);
-        S->init_poisson = nullptr;
+        // what the solve made beyond the stage's own arrays goes back
+        if (S->init_poisson->borrows) {
+            S->init_poisson->release_chunks();
+        } else {
+            gb_poisson_destroy(S->init_poisson);
+            S->init_poisson = nullptr;
+        }
     }
     dsum(S, valid_box(g, CC), w.rhs, 0, 1);
     double sums[3];

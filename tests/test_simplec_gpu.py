@@ -345,3 +345,51 @@ def test_gpu_iteration_graphs_equal_eager_launches(ctx, precision):
     for f in FIELDS:
         assert np.array_equal(out[0][0][f], out[1][0][f]), f
     assert out[0][1] == out[1][1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("restart", [2, 50])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_gpu_initializer_shares_the_correction_solvers_arrays(ctx, precision, restart):
+    """The initializer's projection works in the correction solver's arrays and
+    keeps its solver from call to call: the initial state of a stage that has
+    iterated, and the iterations after it, equal a new stage's bit for bit;
+    so do initial states with other options in between (split coefficients, a
+    projection in FP32 on an FP64 stage, a looser tolerance), with a restart
+    whose vectors the stage does not hold."""
+    from ablsteadyrans_b200 import abi, workloads
+    from ablsteadyrans_b200.simplec import FIELDS
+
+    def stage():
+        import ablsteadyrans_b200 as gb
+        from ablsteadyrans_b200.simplec import DeviceCase, SimplecStage
+        inst = workloads.tile(40, 24, 3, precision=precision)
+        inst.options.poisson.restart = restart
+        J, ax, ay, az, _ = oracle.metrics(inst.grid, inst.z)
+        dc = DeviceCase(inst.grid, inst.z, J, ax, ay, az, inst.nu, inst.gamma_theta, inst.gamma_tke, inst.q, inst.z0map)
+        return SimplecStage(ctx, dc, inst.bc, inst.physics, inst.options), dc
+
+    split = abi.InitOptions.make(alpha_v=0.5)
+    loose = abi.InitOptions.make()
+    loose.poisson.reltol = 1e-4
+    other = abi.InitOptions.make()
+    other.poisson.precision = 1 - precision
+    plain = abi.InitOptions.make()
+
+    def run(st, dc, o):
+        res = st.initialize(o)
+        out = [dc.host(f) for f in FIELDS]
+        for _ in range(2):
+            st.iterate(st.local_dtau(2.0))
+        return out + [dc.host(f) for f in FIELDS], res.poisson_iterations
+
+    used, dc = stage()
+    for o in (plain, split, plain, loose, other, plain):
+        got, its = run(used, dc, o)
+        fresh, dc2 = stage()
+        want, its2 = run(fresh, dc2, o)
+        fresh.close()
+        assert its == its2
+        for n, (a, b) in enumerate(zip(got, want)):
+            assert np.array_equal(a, b), n
+    used.close()
