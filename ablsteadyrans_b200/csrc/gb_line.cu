@@ -37,6 +37,7 @@ struct LineArgs {
     T* __restrict__ ebuf;
     int first;  // dold == 0: no neighbour terms, change against 0
     unsigned long long* change;  // max |dnew - dold| (nullptr: not wanted)
+    unsigned long long* clear;   // a word the sweep sets to 0 for a later one (nullptr: none)
     const T* __restrict__ rfold;  // rhs with the lagged lateral terms folded in (the split sweep)
 };
 
@@ -524,6 +525,13 @@ __device__ __forceinline__ void zline_seg_body(const LineArgs<T>& a, T* __restri
         } else {
             dg[q] = inv_io[o];
             up[q] = cp_io[o];
+        }
+    }
+    if (!FIRST && !PREF) {
+#pragma unroll
+        for (int q = 0; q < L; ++q) {
+            const int64_t ko = static_cast<int64_t>(min(k0 + q, nk - 1)) * g.sz;
+            const int64_t o = o0 + ko;
             const T vxm = a.dold[oxm + ko], vxp = a.dold[oxp + ko], vym = a.dold[oym + ko], vyp = a.dold[oyp + ko];
             const T dxm = hxm ? vxm : T(0);
             const T dxp = hxp ? vxp : T(0);
@@ -618,6 +626,7 @@ __device__ __forceinline__ void zline_seg_body(const LineArgs<T>& a, T* __restri
     __syncthreads();
     {
         T eprev = T(0);
+#pragma unroll 4
         for (int s = 0; s < w; ++s) {
             const int m = s * 32 + lane;
             eprev = carry_e[m] + carry_e[cs + m] * eprev;
@@ -656,6 +665,7 @@ __device__ __forceinline__ void zline_seg_body(const LineArgs<T>& a, T* __restri
     T chg = T(0);
     {
         T x = T(0);
+#pragma unroll 4
         for (int s = W - 1; s > w; --s) {
             const int m = s * 32 + lane;
             x = carry_x[m] + carry_x[cs + m] * x;
@@ -676,6 +686,7 @@ __device__ __forceinline__ void zline_seg_body(const LineArgs<T>& a, T* __restri
             }
         }
     }
+    if (FIRST && a.clear != nullptr && cblock == 0 && me == 0) { *a.clear = 0ull; }
     if (a.change != nullptr) {
         chg = warp_max(chg);
         if (lane == 0) { atomic_max_nonneg(a.change, chg); }
@@ -1005,13 +1016,17 @@ gb_status zline_sweeps_multi(gb_ctx* ctx, const gb_grid& g, int n, const int* lo
         inv[s] = static_cast<T*>(scratch(ctx, kSlotMultiBase + 3 * s + 1, sizeof(T) * vol));
         cpr[s] = static_cast<T*>(scratch(ctx, kSlotMultiBase + 3 * s + 2, sizeof(T) * vol));
         if (!tmp[s] || !inv[s] || !cpr[s]) { return GB_OOM; }
-        if (change_words != nullptr && change_words[s] != nullptr) {
-            cudaMemsetAsync(change_words[s], 0, sizeof(unsigned long long), ctx->stream);
-        }
     }
     // the segmented sweep (the default; GB_TUNE_LINE_VARIANT 4 selects the factored one below)
     const int segL = seg_levels(ctx);
     const int segW = seg_warps(max_nk, segL);
+    // the change words start from 0: set by the first of several segmented sweeps
+    // (a memset is a launch of its own), else here
+    const bool sweep_clears = ctx->tune[GB_TUNE_LINE_VARIANT] != 4 && segW > 0 && sweeps > 1
+                              && ctx->tune[GB_TUNE_LINE_FIRST] != 2;
+    for (int s = 0; s < n && !sweep_clears && change_words != nullptr; ++s) {
+        if (change_words[s] != nullptr) { cudaMemsetAsync(change_words[s], 0, sizeof(unsigned long long), ctx->stream); }
+    }
     if (ctx->tune[GB_TUNE_LINE_VARIANT] != 4 && segW > 0) {
         const dim3 block(32, segW);
         int max_cols = 0;
@@ -1072,6 +1087,7 @@ gb_status zline_sweeps_multi(gb_ctx* ctx, const gb_grid& g, int n, const int* lo
                 a.dnew = buf[(sweeps - 1 - k) & 1];
                 a.first = (k == 0) ? 1 : 0;
                 a.change = (k == sweeps - 1 && change_words != nullptr) ? change_words[s] : nullptr;
+                a.clear = (k == 0 && sweep_clears && change_words != nullptr) ? change_words[s] : nullptr;
                 a.rfold = fold[s];
                 m.inv[s] = inv[s];
                 m.cp[s] = cpr[s];
@@ -1268,6 +1284,31 @@ __global__ void __maxnreg__(batch_reg_cap(L))
     }
 }
 
+//! The batch's increments outside the valid points, and its change words, set
+//! to 0 (a warp per row; blockIdx.y the system): one launch where a memset a
+//! system wrote every point (12 tiles' u, v and w systems: 36 launches and
+//! 370 MB).
+template <typename T>
+__global__ void __launch_bounds__(256) zline_batch_ghosts_kernel(const __grid_constant__ BatchLineParams<T> p)
+{
+    const BatchLineSys<T>& d = p.sys[blockIdx.y];
+    const gb_grid& g = d.a.g;
+    const int lane = threadIdx.x & 31;
+    const int sy = static_cast<int>(g.sy), sz = static_cast<int>(g.sz);
+    const int per_plane = sz / sy, rows = static_cast<int>(d.a.cs / sz) * per_plane;
+    for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += (gridDim.x * blockDim.x) >> 5) {
+        const int kk = row / per_plane, jj = row - kk * per_plane;
+        const int k = kk - g.ng, j = jj - g.ng;
+        T* r = d.buf[0] + static_cast<int64_t>(kk) * sz + static_cast<int64_t>(jj) * sy;
+        const int n = (jj == per_plane - 1) ? sz - jj * sy : sy;  // the last row to the plane's end
+        // a valid row's ends: ng below its ni points, the rest above them
+        const bool valid = k >= 0 && k < d.a.nk && j >= 0 && j < d.a.nj;
+        for (int i = lane; i < (valid ? g.ng : n); i += 32) { r[i] = T(0); }
+        for (int i = g.ng + d.a.ni + lane; valid && i < n; i += 32) { r[i] = T(0); }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) { *d.change = 0ull; }
+}
+
 template <typename T, bool FIRST, int L>
 cudaError_t launch_seg_batch(const BatchLineParams<T>& sys, int warps, int sweep, int sweeps, cudaStream_t stream)
 {
@@ -1373,8 +1414,11 @@ gb_status zline_sweeps_batch(gb_ctx* ctx, int n, const gb_grid* grids, const int
             pr.nsys = local + 1;
         }
     }
-    for (int s = 0; s < n; ++s) { cudaMemsetAsync(delta[s], 0, sizeof(T) * volume(grids[s]), ctx->stream); }
-    cudaMemsetAsync(d_words, 0, sizeof(unsigned long long) * n, ctx->stream);
+    // the increments' ghosts (the sweeps write every valid point) and the change words
+    for (const BatchLineParams<T>& pr : params) {
+        zline_batch_ghosts_kernel<T><<<dim3(2 * ctx->num_sms, pr.nsys), 256, 0, ctx->stream>>>(pr);
+        ++ctx->launches;
+    }
     for (int k = 0; k < sweeps; ++k) {
         for (size_t q = 0; q < launches.size(); ++q) {
             Span span(ctx, GB_KERNEL_LINE_SWEEP);

@@ -2075,8 +2075,8 @@ gb_status line_solve(gb_simplec* S, int loc, const double* A, const double* ap, 
 {
     gb_ctx* ctx = S->ctx;
     const int64_t vol = volume(S->g);
-    cudaMemsetAsync(delta, 0, sizeof(double) * vol, ctx->stream);
     if (S->opt.line_sweep == 1) {  // steady.sweep = lusgs (FP64 in either precision)
+        cudaMemsetAsync(delta, 0, sizeof(double) * vol, ctx->stream);
         return zline_lusgs(ctx, S->g, loc, A, ap, rhs, S->opt.zline_sweeps, S->opt.line_alternate, delta,
                            dword(ctx, word));
     }
@@ -2089,7 +2089,6 @@ gb_status line_solve(gb_simplec* S, int loc, const double* A, const double* ap, 
     k_convert<float><<<nb, 256, 0, ctx->stream>>>(S->w.ap32, ap, vol);
     k_convert<float><<<nb, 256, 0, ctx->stream>>>(S->w.rhs32, rhs, vol);
     ctx->launches += 3;
-    cudaMemsetAsync(S->w.delta32, 0, sizeof(float) * vol, ctx->stream);
     gb_status st = zline_sweeps<float>(ctx, S->g, loc, S->w.A32, S->w.ap32, S->w.rhs32, S->opt.zline_sweeps,
                                        S->w.delta32, dword(ctx, word), LineScratch::automatic);
     const float* d32 = S->w.delta32;
@@ -2117,11 +2116,10 @@ gb_status line_solve_multi(gb_simplec* S, int n, const int* locs, double* const*
         }
         return GB_OK;
     }
+    // (the sweeps write every valid point of delta and read none of it before;
+    // its users read valid points only, so it need not be zeroed)
     unsigned long long* cw[3];
-    for (int s = 0; s < n; ++s) {
-        cudaMemsetAsync(delta[s], 0, sizeof(double) * vol, ctx->stream);
-        cw[s] = dword(ctx, words[s]);
-    }
+    for (int s = 0; s < n; ++s) { cw[s] = dword(ctx, words[s]); }
     if (S->opt.precision == 0) {
         const double* Ac[3] = {A[0], n > 1 ? A[1] : nullptr, n > 2 ? A[2] : nullptr};
         const double* apc[3] = {ap[0], n > 1 ? ap[1] : nullptr, n > 2 ? ap[2] : nullptr};
@@ -2139,7 +2137,6 @@ gb_status line_solve_multi(gb_simplec* S, int n, const int* locs, double* const*
         k_convert<float><<<nb, 256, 0, ctx->stream>>>(w.ap32m[s], ap[s], vol);
         k_convert<float><<<nb, 256, 0, ctx->stream>>>(w.rhs32m[s], rhs[s], vol);
         ctx->launches += 3;
-        cudaMemsetAsync(w.delta32m[s], 0, sizeof(float) * vol, ctx->stream);
         A32[s] = w.A32m[s];
         ap32[s] = w.ap32m[s];
         r32[s] = w.rhs32m[s];
