@@ -8,6 +8,8 @@
 
 #include "gb_common.cuh"
 
+#include <algorithm>
+
 namespace gb {
 namespace st {
 
@@ -109,28 +111,35 @@ inline Box valid_box(const gb_grid& g, int t)
     return Box{{0, 0, 0}, {g.nx - 1 + (t & 1), g.ny - 1 + ((t >> 1) & 1), g.nz - 1 + ((t >> 2) & 1)}};
 }
 
+//! One thread per point: the points of a plane along the grid's x (their row
+//! by one multiply and shift, FastDiv), the planes along its y and z. A linear index
+//! over the box took two 64-bit divisions a point, which in the pointwise
+//! kernels (an outer iteration has some hundred) were more instructions than
+//! the points' own work.
 template <typename F>
-__global__ void k_box(Box b, F f)
+__global__ void k_box(Box b, FastDiv row, F f)
 {
     pdl_entry();
-    const int64_t n = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    const int nx = b.hi[0] - b.lo[0] + 1, ny = b.hi[1] - b.lo[1] + 1;
-    if (n >= b.count()) { return; }
-    const int i = b.lo[0] + static_cast<int>(n % nx);
-    const int j = b.lo[1] + static_cast<int>((n / nx) % ny);
-    const int k = b.lo[2] + static_cast<int>(n / (static_cast<int64_t>(nx) * ny));
-    f(i, j, k);
+    const int n = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (n >= row.d * (b.hi[1] - b.lo[1] + 1)) { return; }
+    const int jj = row.quot(n);
+    const int i = b.lo[0] + n - jj * row.d, j = b.lo[1] + jj;
+    const int k = b.lo[2] + static_cast<int>(blockIdx.y + blockIdx.z * gridDim.y);
+    if (k <= b.hi[2]) { f(i, j, k); }
 }
 
 //! One thread per point of b (i fastest), on the context's stream.
 template <typename F>
 void for_box(gb_ctx* ctx, const Box& b, F f, int family = -1)
 {
-    const int64_t n = b.count();
-    if (n <= 0) { return; }
+    if (b.count() <= 0) { return; }
+    const int row = b.hi[0] - b.lo[0] + 1;
+    const int64_t plane = static_cast<int64_t>(row) * (b.hi[1] - b.lo[1] + 1);
+    const int planes = b.hi[2] - b.lo[2] + 1, py = std::min(planes, 65535);
     if (family >= 0) { span_begin(ctx, family); }
-    launch_pdl(ctx->tune[GB_TUNE_PDL] != 1, k_box<F>, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0,
-               ctx->stream, b, f);
+    launch_pdl(ctx->tune[GB_TUNE_PDL] != 1, k_box<F>,
+               dim3(static_cast<unsigned>((plane + 255) / 256), py, (planes + py - 1) / py), dim3(256), 0, ctx->stream,
+               b, FastDiv(row), f);
     if (family >= 0) { span_end(ctx); }
     ++ctx->launches;
 }
