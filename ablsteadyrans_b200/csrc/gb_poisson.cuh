@@ -293,8 +293,8 @@ __device__ __forceinline__ T adotx_cell(const gb_grid& g, const PBC& b, int i, i
 template <typename T>
 __device__ __forceinline__ void line_tridiag(const gb_grid& g, const PBC& b, const T* __restrict__ AX,
                                              const T* __restrict__ AY, const T* __restrict__ AZ,
-                                             const T* __restrict__ Jc, const T* __restrict__ zp, int i, int j, int k,
-                                             T& D, T& C, T& U)
+                                             const T* __restrict__ Jc, const T* __restrict__ zp,
+                                             const T* __restrict__ hz, int i, int j, int k, T& D, T& C, T& U)
 {
     const T dxinv = static_cast<T>(b.dxinv), dyinv = static_cast<T>(b.dyinv), dzinv = static_cast<T>(b.dzinv);
     T c = T(0);
@@ -310,12 +310,8 @@ __device__ __forceinline__ void line_tridiag(const gb_grid& g, const PBC& b, con
     if (!b.per_y && j == 0 && b.syl < 0) { cyl = T(2) * dyinv; }
     if (!b.per_y && j == g.ny - 1 && b.syh < 0) { cyh = T(2) * dyinv; }
     c -= (myh * AY[at(g, i, j + 1, k)] * cyh + myl * AY[at(g, i, j, k)] * cyl) * dyinv;
-#define Z(a, bb, cc) zp[at(g, a, bb, cc)]
-    const T hzi_hi = T(8) / ((Z(i, j, k + 2) + Z(i + 1, j, k + 2) + Z(i, j + 1, k + 2) + Z(i + 1, j + 1, k + 2))
-                             - (Z(i, j, k) + Z(i + 1, j, k) + Z(i, j + 1, k) + Z(i + 1, j + 1, k)));
-    const T hzi_lo = T(8) / ((Z(i, j, k + 1) + Z(i + 1, j, k + 1) + Z(i, j + 1, k + 1) + Z(i + 1, j + 1, k + 1))
-                             - (Z(i, j, k - 1) + Z(i + 1, j, k - 1) + Z(i, j + 1, k - 1) + Z(i + 1, j + 1, k - 1)));
-#undef Z
+    // 1 / h_zeta of the two z-faces: the mesh ratios (the same quotients, taken once per mesh)
+    const T hzi_hi = hz[at(g, i, j, k + 1)], hzi_lo = hz[at(g, i, j, k)];
     const T mzl = (k != 0) ? T(1) : T(0);
     const T mzh = ((b.zf & TP_ZHI) && k == g.nz - 1) ? T(0) : T(1);
     const T wh = mzh * AZ[at(g, i, j, k + 1)] * hzi_hi * dzinv;

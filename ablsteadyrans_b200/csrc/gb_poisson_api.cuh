@@ -117,6 +117,5 @@ gb_status mesh_metrics(gb_ctx* ctx, const gb_grid& g, const double* z, double* J
                        double* zcc);
 gb_status face_divergence(gb_ctx* ctx, const gb_grid& g, const double* ax, const double* ay, const double* az,
                           const double* J, const double* fx, const double* fy, const double* fz, double* div);
-void multiply_inplace(gb_ctx* ctx, double* a, const double* b, int64_t n);
 
 }  // namespace gb
