@@ -351,8 +351,8 @@ struct SimplecWork {
     double* theta_ref;
     double* conv0;
     double* conv1;
-    double* og;
-    double* level_sum;
+    double* dmask[3];   // each component's Dirichlet points (dirichlet_rows: they depend on the conditions alone)
+    double* level_sum[2];
     double* partial;
     double* sums;
     float* A32;
@@ -423,6 +423,13 @@ struct gb_simplec {
     double lin_speed{1};
     bool lin_ready{false};
     cudaStream_t capture_stream{nullptr};
+    // the side streams and events of launches that do not depend on one another (Branches)
+    static constexpr int kSides = 4;
+    cudaStream_t side[kSides]{};
+    cudaEvent_t fork_ev{nullptr};
+    cudaEvent_t join_ev[kSides]{};
+    int sides{-1};   // -1: not made yet; 0: could not be made
+    bool forked{false};
     cudaGraphExec_t seg_exec[2]{nullptr, nullptr};
     int64_t seg_launches[2]{0, 0};
     uint64_t seg_key[2]{0, 0};
@@ -432,6 +439,11 @@ struct gb_simplec {
 
 gb_simplec::~gb_simplec()
 {
+    for (int n = 0; n < kSides; ++n) {
+        if (side[n]) { cudaStreamDestroy(side[n]); }
+        if (join_ev[n]) { cudaEventDestroy(join_ev[n]); }
+    }
+    if (fork_ev) { cudaEventDestroy(fork_ev); }
     if (poisson) { gb_poisson_destroy(poisson); }
     if (init_poisson) { gb_poisson_destroy(init_poisson); }
     for (void* p : owned) { cudaFree(p); }
@@ -466,6 +478,73 @@ float* fbuf(gb_simplec* S, int64_t n)
     S->owned.push_back(p);
     return static_cast<float*>(p);
 }
+
+// --------------------------------------------------- independent launches ---
+
+//! Launch sequences that do not depend on one another, each on a stream of its
+//! own between a fork and a join: on(b) sends what follows to branch b (0: the
+//! context's stream), join() makes the context's stream wait for all of them.
+//! Every side stream starts after the work queued before the fork and the
+//! context's stream goes on after the join, so callers see one stream. Under
+//! capture the branches become parallel paths of the graph. A small grid's
+//! launches (32 x 32 x 48: five residual launches of 22 us, each on 96 of 148
+//! SMs and bound by latency) then run side by side, and a large one's fill each
+//! other's last waves. One stream while profiling, with GB_TUNE_GRAPHS = 1
+//! (every kernel alone) and inside another fork.
+class Branches {
+public:
+    explicit Branches(gb_simplec* S) : S_(S), main_(S->ctx->stream)
+    {
+        if (S->forked || S->ctx->profiling || S->ctx->tune[GB_TUNE_GRAPHS] == 1 || !ready()) { return; }
+        open_ = S->forked = cudaEventRecord(S->fork_ev, main_) == cudaSuccess;
+    }
+    Branches(const Branches&) = delete;
+    Branches& operator=(const Branches&) = delete;
+    ~Branches() { join(); }
+    void on(int b)
+    {
+        if (!open_) { return; }
+        if (b > 0 && !(used_ & (1u << b))) {
+            cudaStreamWaitEvent(S_->side[b - 1], S_->fork_ev, 0);
+            used_ |= 1u << b;
+        }
+        S_->ctx->stream = (b > 0) ? S_->side[b - 1] : main_;
+    }
+    //! Branch b alone: the context's stream goes on after what it was sent so far.
+    void join(int b)
+    {
+        if (!open_) { return; }
+        S_->ctx->stream = main_;
+        if (used_ & (1u << b)) {
+            cudaEventRecord(S_->join_ev[b - 1], S_->side[b - 1]);
+            cudaStreamWaitEvent(main_, S_->join_ev[b - 1], 0);
+        }
+    }
+    void join()
+    {
+        if (!open_) { return; }
+        for (int b = 1; b <= gb_simplec::kSides; ++b) { join(b); }
+        open_ = S_->forked = false;
+    }
+
+private:
+    bool ready()
+    {
+        if (S_->sides >= 0) { return S_->sides > 0; }
+        bool ok = cudaEventCreateWithFlags(&S_->fork_ev, cudaEventDisableTiming) == cudaSuccess;
+        for (int n = 0; n < gb_simplec::kSides && ok; ++n) {
+            ok = cudaStreamCreateWithFlags(&S_->side[n], cudaStreamNonBlocking) == cudaSuccess
+                 && cudaEventCreateWithFlags(&S_->join_ev[n], cudaEventDisableTiming) == cudaSuccess;
+        }
+        if (!ok) { cudaGetLastError(); }
+        S_->sides = ok ? gb_simplec::kSides : 0;
+        return ok;
+    }
+    gb_simplec* S_;
+    cudaStream_t main_;
+    unsigned used_{0};
+    bool open_{false};
+};
 
 // --------------------------------------------------------- reductions ---
 
@@ -1010,9 +1089,14 @@ void convection(gb_simplec* S, const double* q, double* const* F, int lim, doubl
 {
     const double eps2 = eps * eps;
     double** G = S->w.G;
-    conv_fluxes<T, 0>(S, q, F[0], lim, eps2, G[0]);
-    conv_fluxes<T, 1>(S, q, F[1], lim, eps2, G[1]);
-    conv_fluxes<T, 2>(S, q, F[2], lim, eps2, G[2]);
+    {
+        Branches br(S);
+        conv_fluxes<T, 0>(S, q, F[0], lim, eps2, G[0]);
+        br.on(1);
+        conv_fluxes<T, 1>(S, q, F[1], lim, eps2, G[1]);
+        br.on(2);
+        conv_fluxes<T, 2>(S, q, F[2], lim, eps2, G[2]);
+    }
     flux_divergence<T>(S, G[0], G[1], G[2], out, 0);
     if (bounded) { subtract_transport_divergence<T>(S, q, F[0], F[1], F[2], out); }
 }
@@ -1241,8 +1325,8 @@ __global__ void __launch_bounds__(256, 4) k_momentum_stress(const StressArgs a)
     if (NP == 3 && in[2]) { a.G[2][o] = flux(I2{}, I2{}); }
 }
 
-//! The nine momentum diffusive fluxes into w.Gd in four launches.
-void momentum_stress(gb_simplec* S, const gb_state& q)
+//! The nine momentum diffusive fluxes into w.Gd in four launches (a branch each).
+void momentum_stress(gb_simplec* S, const gb_state& q, Branches& br)
 {
     const gb_grid g = S->g;
     double** Gd = S->w.Gd;
@@ -1280,9 +1364,13 @@ void momentum_stress(gb_simplec* S, const gb_state& q)
         span_end(S->ctx);
         ++S->ctx->launches;
     };
+    br.on(0);
     launch(std::integral_constant<int, CC>{}, 0, 0, 1, 1, 2, 2);
+    br.on(1);
     launch(std::integral_constant<int, XF ^ YF>{}, 0, 1, 1, 0, -1, -1);
+    br.on(2);
     launch(std::integral_constant<int, XF ^ ZF>{}, 0, 2, 2, 0, -1, -1);
+    br.on(3);
     launch(std::integral_constant<int, YF ^ ZF>{}, 1, 2, 2, 1, -1, -1);
 }
 
@@ -1685,21 +1773,44 @@ void simplec_residual(gb_simplec* S, const gb_state& q, double** R)
     gb_ctx* ctx = S->ctx;
     const gb_grid g = S->g;
     const int64_t vol = volume(g);
-    for (int n = 0; n < 6; ++n) { cudaMemsetAsync(R[n], 0, sizeof(double) * vol, ctx->stream); }
-    // the closure's fields and the wall state at q (Residual.cpp:166-176, 205-208)
-    if (S->ph.closure) {
-        turb_closure(ctx, g, S->bc, S->ph, q, S->z, S->dist, S->mesh.z0, S->cf, S->has_hist ? S->nut_hist : nullptr);
+    // (every valid point is written below; the stage's own residuals' ghosts are
+    // zero from their allocation on)
+    for (int n = 0; n < 6; ++n) {
+        if (R[n] != S->w.R[n]) { cudaMemsetAsync(R[n], 0, sizeof(double) * vol, ctx->stream); }
     }
-    if (S->wall) { turb_surface_state(ctx, g, S->bc, S->ph, q, S->z, S->mesh.z0, S->ssr, dword(ctx, W_SURFACE_BAD)); }
+    // the closure's fields and the wall state at q (Residual.cpp:166-176, 205-208)
     double** F = S->w.F;
-    transport_fluxes(S, q, F[0], F[1], F[2]);
+    {
+        Branches br(S);
+        if (S->ph.closure) {
+            turb_closure(ctx, g, S->bc, S->ph, q, S->z, S->dist, S->mesh.z0, S->cf, S->has_hist ? S->nut_hist : nullptr);
+        }
+        br.on(1);
+        if (S->wall) { turb_surface_state(ctx, g, S->bc, S->ph, q, S->z, S->mesh.z0, S->ssr, dword(ctx, W_SURFACE_BAD)); }
+        br.on(2);
+        transport_fluxes(S, q, F[0], F[1], F[2]);
+        br.on(3);
+        velocity_divergence(S, q.u, q.v, q.w, R[3]);
+    }
     const gb_physics& ph = S->ph;
     const bool fused = ctx->tune[GB_TUNE_RESIDUAL] != 1;
     if (fused) {
-        momentum_stress(S, q);
-        fused_residual<0>(S, q, R[0]);
+        {
+            Branches br(S);
+            momentum_stress(S, q, br);
+            br.on(4);
+            fused_residual<4>(S, q, R[5]);
+            if (S->wall) { turb_apply_wall_k(ctx, g, S->bc, S->ssr, q.tke, R[5]); }
+        }
+        Branches br(S);
+        br.on(1);
+        fused_residual<3>(S, q, R[4]);
+        br.on(2);
         fused_residual<1>(S, q, R[1]);
+        br.on(3);
         fused_residual<2>(S, q, R[2]);
+        br.on(0);
+        fused_residual<0>(S, q, R[0]);
     } else {
         convection<XF>(S, q.u, F, ph.limiter, ph.smooth_eps_velocity, false, R[0]);
         convection<YF>(S, q.v, F, ph.limiter, ph.smooth_eps_velocity, false, R[1]);
@@ -1710,18 +1821,14 @@ void simplec_residual(gb_simplec* S, const gb_state& q, double** R)
         add_pressure_gradient(S, q.p, R[0], R[1], R[2]);
     }
     forcing(S, q, R);
-    velocity_divergence(S, q.u, q.v, q.w, R[3]);
-    if (fused) {
-        fused_residual<3>(S, q, R[4]);
-        fused_residual<4>(S, q, R[5]);
-    } else {
+    if (!fused) {
         convection<CC>(S, q.theta, F, ph.limiter, ph.smooth_eps_theta, false, R[4]);
         scalar_diffusion_subtract(S, q.theta, S->dfe.gamma_theta, R[4], 2);
         convection<CC>(S, q.tke, F, GB_LIMITER_UPWIND, 1e-5, true, R[5]);
         scalar_diffusion_subtract(S, q.tke, S->dfe.gamma_tke, R[5], 3);
         if (S->ph.closure) { turb_k_sources(ctx, g, S->cf, R[5]); }
+        if (S->wall) { turb_apply_wall_k(ctx, g, S->bc, S->ssr, q.tke, R[5]); }
     }
-    if (S->wall) { turb_apply_wall_k(ctx, g, S->bc, S->ssr, q.tke, R[5]); }
     add_damping(S, q, R);
     apply_rows(S, q, R);
     seam_sync<double>(ctx, g, XF, R[0]);
@@ -2183,7 +2290,7 @@ void residual_sums(gb_simplec* S, const gb_state& q)
     dsum_many(S, P);
 }
 
-gb_status momentum_predictor(gb_simplec* S, const gb_state& q, double** R)
+gb_status momentum_predictor(gb_simplec* S, const gb_state& q, double** R, bool monitors = false)
 {
     gb_ctx* ctx = S->ctx;
     const gb_grid g = S->g;
@@ -2193,14 +2300,26 @@ gb_status momentum_predictor(gb_simplec* S, const gb_state& q, double** R)
     const double fs = S->ph.coriolis ? 4 * 3.14159265358979323846 * std::sin(S->ph.latitude * 3.14159265358979323846 / 180)
                                          / S->ph.rotation_period
                                      : 0.0;
+    // each component's rows on a branch, theta's (the buoyancy coupling's) on a fourth
+    const bool buoyant = S->ph.gravity > 0;
+    Branches br(S);
+    if (monitors) {
+        br.on(4);
+        residual_sums(S, q);
+        dmax_velocity(S, q.u, q.v, q.w, W_MON_U);
+    }
+    if (buoyant) {
+        br.on(3);
+        simplec_implicit_rows(S, F_THETA, w.F, w.At);
+    }
     for (int c = 0; c < 3; ++c) {
+        br.on(c);
         const int t = 1 << c;
         simplec_implicit_rows(S, c, w.F, w.Am[c]);
-        dirichlet_rows(S, c, t, w.mask);
         double* ap = w.ap[c];
         double* dd = w.dd[c];
         const double* A = w.Am[c];
-        const double* mask = w.mask;
+        const double* mask = w.dmask[c];
         const double* dt = w.dtf[c];
         const double* Rc = R[c];
         double* rhs = w.rhsm[c];
@@ -2249,13 +2368,11 @@ gb_status momentum_predictor(gb_simplec* S, const gb_state& q, double** R)
                 Box b = valid_box(g, to);
                 if (per_o) { b.hi[d_o] -= 1; }
                 Span span(ctx, GB_KERNEL_VECTOR);
-                k_level_mean<<<g.nz, kLevelThreads, 0, ctx->stream>>>(g, b, other, npts_level, w.level_sum);
+                k_level_mean<<<g.nz, kLevelThreads, 0, ctx->stream>>>(g, b, other, npts_level, w.level_sum[c]);
                 ++ctx->launches;
             }
-            double* mean = w.level_sum;
-            // the periodic images of the other residual (one ghost) for the four-face mean
-            cudaMemcpyAsync(w.og, other, sizeof(double) * cs, cudaMemcpyDeviceToDevice, ctx->stream);
-            double* og = w.og;
+            const double* mean = w.level_sum[c];
+            const double* og = other;  // read with its periodic images for the four-face mean
             const bool px = g.periodic_x, py = g.periodic_y;
             const double relax = S->opt.rotation_relax;
             const bool per_c = is_per(g, c);
@@ -2298,9 +2415,10 @@ gb_status momentum_predictor(gb_simplec* S, const gb_state& q, double** R)
                 rhs[o] += ((cc == 0) ? -fs : fs) * (tau_c * m + tau_own * (avg - m));
             }, GB_KERNEL_COEFS);
         }
-        if (c == 2 && S->ph.gravity > 0) {
+        if (c == 2 && buoyant) {
+            br.join(2);
+            br.join(3);
             const double gt = S->ph.gravity / S->ph.theta0;
-            simplec_implicit_rows(S, F_THETA, w.F, w.At);
             const double* At = w.At;
             const double* th = q.theta;
             const double* Rt = R[4];
@@ -2323,13 +2441,17 @@ gb_status momentum_predictor(gb_simplec* S, const gb_state& q, double** R)
             }, GB_KERNEL_COEFS);
         }
     }
+    br.join();
     // the three systems are independent: one batched solve
     const int locs[3] = {XF, YF, ZF};
     const int words[3] = {W_LAST_U, W_LAST_V, W_LAST_W};
     gb_status st = line_solve_multi(S, 3, locs, w.Am, w.ap, w.rhsm, w.deltam, words);
     if (st != GB_OK) { return st; }
+    Branches up(S);
+    up.on(3);
     dmax_velocity(S, w.deltam[0], w.deltam[1], w.deltam[2], W_MAX_DU);
     for (int c = 0; c < 3; ++c) {
+        up.on(c);
         const int t = 1 << c;
         double* qc = comps[c];
         const double* delta = w.deltam[c];
@@ -2342,13 +2464,16 @@ gb_status momentum_predictor(gb_simplec* S, const gb_state& q, double** R)
 }
 
 //! pressure_correction's first part: beta = 1/d and the keep masks, div u*,
-//! the monitors, the solver's coefficients (no host synchronisation).
-gb_status pressure_prelude(gb_simplec* S, const gb_state& q, const double* source = nullptr)
+//! the monitors, the solver's coefficients (no host synchronisation); with
+//! theta_conv also theta's convection at q with the stage's transport.
+gb_status pressure_prelude(gb_simplec* S, const gb_state& q, const double* source = nullptr, double* theta_conv = nullptr)
 {
     gb_ctx* ctx = S->ctx;
     const gb_grid g = S->g;
     SimplecWork& w = S->w;
+    Branches br(S);
     for (int c = 0; c < 3; ++c) {
+        br.on(c);
         const double* dd = w.dd[c];
         double* beta = w.beta[c];
         double* keep = w.keep[c];
@@ -2359,6 +2484,7 @@ gb_status pressure_prelude(gb_simplec* S, const gb_state& q, const double* sourc
             keep[o] = on ? 1.0 : 0.0;
         }, GB_KERNEL_COEFS);
     }
+    br.on(3);
     velocity_divergence(S, q.u, q.v, q.w, w.rhs);
     if (source != nullptr) {
         // the Newton preconditioner's continuity rows: div(du) = r_p
@@ -2378,6 +2504,12 @@ gb_status pressure_prelude(gb_simplec* S, const gb_state& q, const double* sourc
         P.n = 4;
         dmax_many(S, P);
     }
+    if (theta_conv != nullptr) {
+        br.on(4);
+        convection<CC>(S, q.theta, w.F, S->ph.limiter, S->ph.smooth_eps_theta, false, theta_conv);
+    }
+    br.join(1);
+    br.join(2);
     return poisson_set_coeffs(S->poisson, S->mesh.ax, S->mesh.ay, S->mesh.az, w.beta[0], w.beta[1], w.beta[2]);
 }
 
@@ -2421,6 +2553,8 @@ gb_status pressure_finish(gb_simplec* S, const gb_state& q)
     const double alpha = S->opt.alpha_p;
     double* p = q.p;
     const double* phi = w.phi;
+    Branches br(S);
+    br.on(1);
     for_box(ctx, valid_box(g, CC), [=] __device__(int i, int j, int k) {
         const int64_t o = at(g, i, j, k);
         p[o] += alpha * phi[o];
@@ -2432,6 +2566,7 @@ gb_status pressure_finish(gb_simplec* S, const gb_state& q)
         P.n = 4;
         dmax_many(S, P);
     }
+    br.on(0);
     omega_from_w(S, q.u, q.v, q.w, w.om);
     double* tgt[3] = {q.u, q.v, w.om};
     for (int c = 0; c < 3; ++c) {
@@ -2559,7 +2694,9 @@ gb_status scalar_sweeps(gb_simplec* S, const gb_state& q, const double* dtau, bo
     const int eqs[2] = {F_THETA, F_TKE};
     double* fields[2] = {q.theta, q.tke};
     const double* Rq[2] = {w.R[4], w.R[5]};
+    Branches br(S);
     for (int e = 0; e < 2; ++e) {
+        br.on(e);
         simplec_implicit_rows(S, eqs[e], w.F, w.Am[e]);
         double* rhs = w.rhsm[e];
         double* ap = w.ap[e];
@@ -2571,14 +2708,18 @@ gb_status scalar_sweeps(gb_simplec* S, const gb_state& q, const double* dtau, bo
             ap[o] = 1.0 / dtau[o] + A[GB_COEF_P * cs + o];
         }, GB_KERNEL_COEFS);
     }
+    br.join();
     const int locs[2] = {CC, CC};
     const int words[2] = {W_LAST_TH, W_LAST_K};
     gb_status st = line_solve_multi(S, 2, locs, w.Am, w.ap, w.rhsm, w.deltam, words);
     if (st != GB_OK) { return st; }
     const int wmax[2] = {W_MAX_DTH, W_MAX_DK};
     unsigned long long* count = dword(ctx, W_CLIPPED);
+    Branches up(S);
     for (int e = 0; e < 2; ++e) {
+        up.on(2 + e);
         dmax(S, valid_box(g, CC), w.deltam[e], nullptr, wmax[e]);
+        up.on(e);
         const double* delta = w.deltam[e];
         double* field = fields[e];
         const bool do_clip = (eqs[e] == F_TKE) && clip;
@@ -2617,14 +2758,12 @@ gb_status simplec_iterate(gb_simplec* S, const gb_state& q, const double* dtau, 
     if (S->ph.closure) {
         cudaMemcpyAsync(S->nu_dtau, S->cf[kClosureNu], sizeof(double) * volume(g), cudaMemcpyDeviceToDevice, ctx->stream);
     }
-    residual_sums(S, q);
-    dmax_velocity(S, q.u, q.v, q.w, W_MON_U);
-    transport_fluxes(S, q, w.F[0], w.F[1], w.F[2]);
     face_dtau(S, dtau, w.dtf);
-    gb_status s1 = momentum_predictor(S, q, w.R);
+    // (the transport fluxes at q are the residual's)
+    gb_status s1 = momentum_predictor(S, q, w.R, true);
     if (s1 != GB_OK) { return s1; }
     fill_ghosts_into(S, q, S->sst);
-    return pressure_prelude(S, q);
+    return pressure_prelude(S, q, nullptr, w.conv0);
     });
     if (st != GB_OK) { return st; }
     if ((st = pressure_solve(S, info)) != GB_OK) { return st; }
@@ -2632,7 +2771,6 @@ gb_status simplec_iterate(gb_simplec* S, const gb_state& q, const double* dtau, 
     st = run_segment(S, 1, key, [&]() -> gb_status {
     gb_status s2 = pressure_finish(S, q);
     if (s2 != GB_OK) { return s2; }
-    convection<CC>(S, q.theta, w.F, S->ph.limiter, S->ph.smooth_eps_theta, false, w.conv0);
     fill_ghosts_into(S, q, S->sst);
     transport_fluxes(S, q, w.F[0], w.F[1], w.F[2]);
     convection<CC>(S, q.theta, w.F, S->ph.limiter, S->ph.smooth_eps_theta, false, w.conv1);
@@ -3614,8 +3752,8 @@ gb_status simplec_build(gb_simplec* S)
     w.theta_ref = dbuf(S, vol);
     w.conv0 = dbuf(S, vol);
     w.conv1 = dbuf(S, vol);
-    w.og = dbuf(S, vol);
-    w.level_sum = dbuf(S, g.nz + 1);
+    for (int n = 0; n < 2; ++n) { w.level_sum[n] = dbuf(S, g.nz + 1); }
+    for (int n = 0; n < 3; ++n) { w.dmask[n] = dbuf(S, vol); }
     w.partial = dbuf(S, static_cast<int64_t>(kRedBlocks) * (SUM_LEVEL + g.nz + 1));
     w.sums = dbuf(S, SUM_LEVEL + g.nz + 1);
     if (S->opt.precision == 1) {
@@ -3694,6 +3832,7 @@ gb_status simplec_build(gb_simplec* S)
         p.rt[n] = S->bc.theta_ref_theta[n];
     }
     if (S->ph.gravity > 0) { fill_theta_ref(S); }
+    for (int c = 0; c < 3; ++c) { dirichlet_rows(S, c, kLoc[c], w.dmask[c]); }
     // the Poisson solver of the correction (poisson_bc_from_faces, BoundaryConditions.cpp:362-380)
     int32_t pbc[6];
     for (int f = 0; f < 6; ++f) {

@@ -142,3 +142,45 @@ def test_gpu_implicit_coefficients_per_block_faces_match_per_point(ctx, loc, lev
     for n in range(7):
         scale = max(float(np.abs(out[0][n][v]).max()), 1e-300)
         assert float(np.abs(out[1][n][v] - out[0][n][v]).max()) <= 1e-14 * scale, n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", [0, 1], ids=["inflow-coriolis", "hill-closure-wall"])
+@pytest.mark.parametrize("residual", [0, 1], ids=["fused", "separate"])
+def test_gpu_parallel_branches_equal_one_stream(ctx, which, residual):
+    """Launches that do not depend on one another run on side streams
+    (GB_TUNE_GRAPHS = 1: on one): residual, predictor, correction, both scalar
+    sweeps and an application of the preconditioner give the same bits, twice
+    each (the second call meets the first one's arrays)."""
+    import ablsteadyrans_b200 as gb
+    from ablsteadyrans_b200.simplec import DeviceCase, SimplecStage
+    out = []
+    try:
+        ctx.tune(gb.TUNE_RESIDUAL, residual)
+        for graphs in (1, 0):
+            ctx.tune(gb.TUNE_GRAPHS, graphs)
+            name, case, bc, ph = list(_cases())[which]
+            opts = SimplecOptions.make(pressure_reltol=1e-9, zline_sweeps=3, w_vnn_cap=16.0, tke_floor=1e-3)
+            oracle.fill_ghosts(case, bc, ph)
+            dc = DeviceCase.from_oracle(case)
+            st = SimplecStage(ctx, dc, bc, ph, opts)
+            got = []
+            for _ in range(2):
+                st.fill_ghosts()
+                dt = st.local_dtau(2.0)
+                R = st.residual()
+                got += [r.cpu().numpy() for r in R]
+                got += [a.cpu().numpy() for a in st.precondition([-r for r in R], dt)]
+                st.fill_ghosts()
+                st.momentum_predictor(R, dt)
+                st.pressure_correction()
+                st.scalar_sweep(4, R[4], dt)
+                st.scalar_sweep(5, R[5], dt)
+                got += [dc.host(f) for f in FIELDS]
+            out.append(got)
+            st.close()
+    finally:
+        ctx.tune(gb.TUNE_GRAPHS, 0)
+        ctx.tune(gb.TUNE_RESIDUAL, 0)
+    for n, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a, b), n
