@@ -1222,6 +1222,179 @@ __global__ void k_prolong_add(gb_grid gc, PBC bcb, const T* __restrict__ xc, gb_
     prolong_cell<T>(gc, bcb, xc, gf, xf, i, j, k);
 }
 
+//! All relaxations of the coarsest level where it has at most kCoarseCells
+//! cells: k_coarse_relax's operations with a cell a thread. A colour's phase was
+//! one warp's instructions a column (the operator at P levels a lane with its
+//! 21 coefficients, 15 resolved neighbours and their signs, then the scans). Here
+//! every cell has its thread: the coefficients, neighbour positions and signs
+//! stay in registers over all relaxations, r goes through shared memory, and the
+//! warps below nx ny each run one column's scans, whose multipliers do not depend
+//! on r and are formed once.
+//! 2 x 2 x 48 cells in FP64, 8 relaxations: 42 us with k_coarse_relax, 19 so
+//! (the V-cycle of 32 x 32 x 48: 132 -> 112 us).
+//! Shared memory: the iterate, r, D, 1/m, c' ([k][j][i], 5 * nx ny nz).
+constexpr int kCoarseCells = 512;
+
+template <typename T, int P, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
+    k_coarse_relax_cells(gb_grid g, PBC b, int nrelax, T* x, const T* __restrict__ bv, const T* __restrict__ AX,
+                         const T* __restrict__ AY, const T* __restrict__ AZ, const T* __restrict__ J, MeshRatios<T> m,
+                         const T* __restrict__ TD, const T* __restrict__ TC, const T* __restrict__ TU)
+{
+    pdl_entry();
+    constexpr unsigned kAll = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const int pl = nx * ny, plane = pl * nz;
+    T* xs = reinterpret_cast<T*>(smem_raw);
+    T* sr = xs + plane;
+    T* sd = sr + plane;
+    T* sm = sd + plane;
+    T* sc = sm + plane;
+    for (int n = threadIdx.x; n < plane; n += blockDim.x) {
+        const int i = n % nx, j = (n / nx) % ny, k = n / pl;
+        const int64_t o = at(g, i, j, k);
+        xs[n] = T(0);  // the V-cycle's correction starts from zero
+        sd[n] = TD[o];
+        sm[n] = TC[o];
+        sc[n] = TU[o];
+    }
+    // this thread's cell: the first half of the threads take colour 0, the other colour 1
+    const int half = (nx + 1) / 2, per = half * ny * nz;
+    const int mine = static_cast<int>(threadIdx.x) / per, r0 = static_cast<int>(threadIdx.x) - mine * per;
+    const int j = (r0 / half) % ny, k = r0 / (half * ny), i = 2 * (r0 % half) + ((j + mine) & 1);
+    const bool cell = mine < 2 && i < nx;
+    CellCoefs<T> c{};
+    T bo = T(0);
+    int pos[15];          // the neighbours' places in xs
+    unsigned neg = 0;     // whose sign turns (mirrors across an odd face)
+    constexpr int8_t kOff[15][3] = {{0, 0, 0}, {1, 0, 0}, {-1, 0, 0}, {0, 1, 0}, {0, -1, 0}, {0, 0, 1}, {0, 0, -1},
+                                    {1, 0, 1}, {1, 0, -1}, {-1, 0, 1}, {-1, 0, -1}, {0, 1, 1}, {0, 1, -1},
+                                    {0, -1, 1}, {0, -1, -1}};
+    if (cell) {
+        const int64_t o = at(g, i, j, k);
+        c = load_cell_coefs<T>(g, o, AX, AY, AZ, J, m);
+        bo = bv[o];
+        int im, ip, sim, sip, jm, jp, sjm, sjp;
+        resolve_neighbours(i, nx, b.per_x, b.sxl, b.sxh, im, ip, sim, sip);
+        resolve_neighbours(j, ny, b.per_y, b.syl, b.syh, jm, jp, sjm, sjp);
+        const int cx[3] = {im, i, ip}, cy[3] = {jm * nx, j * nx, jp * nx};
+        const int cz[3] = {((k == 0) ? 0 : k - 1) * pl, k * pl, ((k == nz - 1) ? k : k + 1) * pl};
+        const int sx3[3] = {sim, 1, sip}, sy3[3] = {sjm, 1, sjp};
+        const int sz3[3] = {(k == 0) ? b.szl : 1, 1, (k == nz - 1) ? b.szh : 1};
+#pragma unroll
+        for (int q = 0; q < 15; ++q) {
+            const int a0 = kOff[q][0] + 1, a1 = kOff[q][1] + 1, a2 = kOff[q][2] + 1;
+            pos[q] = cx[a0] + cy[a1] + cz[a2];
+            neg |= (sx3[a0] * sy3[a1] * sz3[a2] < 0) ? (1u << q) : 0u;
+        }
+    }
+    __syncthreads();
+    // the column of this warp: the maps' multipliers over the lane's levels and at each step of the scans
+    const int lane = threadIdx.x & 31, col = threadIdx.x >> 5;
+    const bool solver = col < pl;
+    const int ccolor = ((col % nx) + (col / nx)) & 1;
+    T bf[5], db[5];
+    if (solver) {
+        T be = T(1), de = T(1);
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+            const int kk = lane * P + q;
+            if (kk < nz) { be = (kk == 0) ? T(0) : (-sd[col + kk * pl] * be) * sm[col + kk * pl]; }
+        }
+#pragma unroll
+        for (int q = P - 1; q >= 0; --q) {
+            const int kk = lane * P + q;
+            if (kk < nz) { de = (kk == nz - 1) ? T(0) : -sc[col + kk * pl] * de; }
+        }
+#pragma unroll
+        for (int t = 0; t < 5; ++t) {
+            const int d = 1 << t;
+            bf[t] = be;
+            db[t] = de;
+            const T be2 = __shfl_up_sync(kAll, be, d), de2 = __shfl_down_sync(kAll, de, d);
+            if (lane >= d) { be = be * be2; }
+            if (lane + d < 32) { de = de * de2; }
+        }
+    }
+    for (int s = 0; s < 2 * nrelax; ++s) {
+        const int color = s & 1;
+        if (cell && mine == color) {
+            auto X = [&](int di, int dj, int dk) {
+                // the place of (di, dj, dk) in kOff: a constant where X is called
+                const int q = (dk == 0) ? (di > 0 ? 1 : di < 0 ? 2 : dj > 0 ? 3 : dj < 0 ? 4 : 0)
+                            : (di > 0) ? (dk > 0 ? 7 : 8)
+                            : (di < 0) ? (dk > 0 ? 9 : 10)
+                            : (dj > 0) ? (dk > 0 ? 11 : 12)
+                            : (dj < 0) ? (dk > 0 ? 13 : 14)
+                            : (dk > 0 ? 5 : 6);
+                const T v = xs[pos[q]];
+                return (neg & (1u << q)) ? -v : v;
+            };
+            sr[pos[0]] = (s == 0) ? bo : bo - adotx_coefs<T, true>(g, b, i, j, k, X, c, m.zn);
+        }
+        __syncthreads();
+        if (solver && ccolor == color) {
+            T R[P], D[P], IM[P], CP[P], X0[P];
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                const int n = col + min(lane * P + q, nz - 1) * pl;
+                R[q] = sr[n];
+                D[q] = sd[n];
+                IM[q] = sm[n];
+                CP[q] = sc[n];
+                X0[q] = xs[n];
+            }
+            // e_k = (r_k - D_k e_{k-1}) / m_k over this lane's levels as e = al + be e_in, scanned over the lanes
+            T al = T(0);
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                const int kk = lane * P + q;
+                if (kk < nz) { al = (kk == 0) ? R[q] * IM[q] : (R[q] - D[q] * al) * IM[q]; }
+            }
+#pragma unroll
+            for (int t = 0; t < 5; ++t) {
+                const T al2 = __shfl_up_sync(kAll, al, 1 << t);
+                if (lane >= (1 << t)) { al = al + bf[t] * al2; }
+            }
+            T ep = __shfl_up_sync(kAll, al, 1);
+            if (lane == 0) { ep = T(0); }
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                const int kk = lane * P + q;
+                if (kk < nz) {
+                    ep = (kk == 0) ? R[q] * IM[q] : (R[q] - D[q] * ep) * IM[q];
+                    R[q] = ep;
+                }
+            }
+            // x_k = e_k - c'_k x_{k+1} over this lane's levels as x = ga + de x_in
+            T ga = T(0);
+#pragma unroll
+            for (int q = P - 1; q >= 0; --q) {
+                const int kk = lane * P + q;
+                if (kk < nz) { ga = (kk == nz - 1) ? R[q] : R[q] - CP[q] * ga; }
+            }
+#pragma unroll
+            for (int t = 0; t < 5; ++t) {
+                const T ga2 = __shfl_down_sync(kAll, ga, 1 << t);
+                if (lane + (1 << t) < 32) { ga = ga + db[t] * ga2; }
+            }
+            T xk = __shfl_down_sync(kAll, ga, 1);
+            if (lane == 31) { xk = T(0); }
+#pragma unroll
+            for (int q = P - 1; q >= 0; --q) {
+                const int kk = lane * P + q;
+                if (kk < nz) {
+                    xk = (kk == nz - 1) ? R[q] : R[q] - CP[q] * xk;
+                    xs[col + kk * pl] = X0[q] + xk;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    for (int n = threadIdx.x; n < plane; n += blockDim.x) { x[at(g, n % nx, (n / nx) % ny, n / pl)] = xs[n]; }
+}
+
 //! All relaxations of the coarsest level in ONE block. On a level of a few
 //! columns every launch is latency, and the coarsest level takes nu_coarse
 //! relaxations: here the level's iterate and its columns' line factors stay
@@ -2279,11 +2452,23 @@ void vcycle(gb_poisson* P, PoissonLevels<T>& L, int l)
                        static_cast<const T*>(L.AX[l]), static_cast<const T*>(L.AY[l]), static_cast<const T*>(L.AZ[l]), \
                        static_cast<const T*>(L.J[l]), L.ratios(l), static_cast<const T*>(L.TD[l]), \
                        static_cast<const T*>(L.TC[l]), static_cast<const T*>(L.TU[l])
-            switch (pl) {
-            case 1: launch_pdl(pdl, k_coarse_relax<T, 1>, dim3(1), dim3(256), smem, ctx->stream, GB_COARSE_ARGS); break;
-            case 2: launch_pdl(pdl, k_coarse_relax<T, 2>, dim3(1), dim3(256), smem, ctx->stream, GB_COARSE_ARGS); break;
-            case 3: launch_pdl(pdl, k_coarse_relax<T, 3>, dim3(1), dim3(256), smem, ctx->stream, GB_COARSE_ARGS); break;
-            default: launch_pdl(pdl, k_coarse_relax<T, 4>, dim3(1), dim3(256), smem, ctx->stream, GB_COARSE_ARGS); break;
+            // a cell a thread where the block has a thread for each, and a warp for each column's scans
+            const int cells = 2 * ((g.nx + 1) / 2) * g.ny * g.nz;
+            const int threads = (std::max(cells, 32 * g.nx * g.ny) + 31) / 32 * 32;
+            if (threads <= kCoarseCells) {
+                const size_t smem5 = static_cast<size_t>(5) * g.nx * g.ny * g.nz * sizeof(T);
+                // (up to 256 threads with the registers the FP64 coefficients want: no spills)
+                constexpr int A = kCoarseCells / 2, B = kCoarseCells;
+                const bool few = threads <= A;
+                auto kern = (pl == 1) ? (few ? k_coarse_relax_cells<T, 1, A> : k_coarse_relax_cells<T, 1, B>)
+                          : (pl == 2) ? (few ? k_coarse_relax_cells<T, 2, A> : k_coarse_relax_cells<T, 2, B>)
+                          : (pl == 3) ? (few ? k_coarse_relax_cells<T, 3, A> : k_coarse_relax_cells<T, 3, B>)
+                                      : (few ? k_coarse_relax_cells<T, 4, A> : k_coarse_relax_cells<T, 4, B>);
+                launch_pdl(pdl, kern, dim3(1), dim3(threads), smem5, ctx->stream, GB_COARSE_ARGS);
+            } else {
+                auto kern = (pl == 1) ? k_coarse_relax<T, 1> : (pl == 2) ? k_coarse_relax<T, 2>
+                          : (pl == 3) ? k_coarse_relax<T, 3> : k_coarse_relax<T, 4>;
+                launch_pdl(pdl, kern, dim3(1), dim3(256), smem, ctx->stream, GB_COARSE_ARGS);
             }
 #undef GB_COARSE_ARGS
             ++ctx->launches;

@@ -151,6 +151,25 @@ __device__ __forceinline__ T ground_flux_dir(const gb_grid& g, int i, int j, XA&
     return -pz_lo;
 }
 
+//! The operator's 21 coefficients at one cell: the mesh ratios and the
+//! premultiplied areas of its faces and edges, J.
+template <typename T>
+struct CellCoefs {
+    T rxhh, rxhl, rxlh, rxll, ryhh, ryhl, rylh, ryll, hzh, hzl, sxh, sxl, syh, syl;
+    T axh, axl, ayh, ayl, azh, azl, J;
+};
+
+template <typename T>
+__device__ __forceinline__ CellCoefs<T> load_cell_coefs(const gb_grid& g, int64_t o, const T* __restrict__ axa,
+                                                        const T* __restrict__ aya, const T* __restrict__ aza,
+                                                        const T* __restrict__ Jc, const MeshRatios<T>& m)
+{
+    const int sy = static_cast<int>(g.sy), sz = static_cast<int>(g.sz);
+    return CellCoefs<T>{m.rx[o + 1 + sz], m.rx[o + 1], m.rx[o + sz], m.rx[o], m.ry[o + sy + sz], m.ry[o + sy],
+                        m.ry[o + sz], m.ry[o], m.hz[o + sz], m.hz[o], m.sx[o + sz], m.sx[o], m.sy[o + sz], m.sy[o],
+                        axa[o + 1], axa[o], aya[o + sy], aya[o], aza[o + sz], aza[o], Jc[o]};
+}
+
 //! The terrain operator at cell (i, j, k) with the iterate's 15 values read by
 //! X(di, dj, dk): terrpoisson_adotx (ERF_TerrainPoisson_3D_K.H:316-530) with
 //! the premultiplied areas a beta and the zero-flux mask (MASKS: the cell may
@@ -158,9 +177,8 @@ __device__ __forceinline__ T ground_flux_dir(const gb_grid& g, int i, int j, XA&
 //! operations in the same order on the same values, without its ~19
 //! divisions per cell.
 template <typename T, bool MASKS, typename XA>
-__device__ __forceinline__ T adotx_body(const gb_grid& g, const PBC& b, int i, int j, int k, int64_t o, XA&& X,
-                                        const T* __restrict__ axa, const T* __restrict__ aya, const T* __restrict__ aza,
-                                        const T* __restrict__ Jc, const MeshRatios<T>& m)
+__device__ __forceinline__ T adotx_coefs(const gb_grid& g, const PBC& b, int i, int j, int k, XA&& X,
+                                         const CellCoefs<T>& c, const T* __restrict__ zn)
 {
     const T dxinv = static_cast<T>(b.dxinv), dyinv = static_cast<T>(b.dyinv), dzinv = static_cast<T>(b.dzinv);
     const T h = T(0.5);
@@ -168,52 +186,51 @@ __device__ __forceinline__ T adotx_body(const gb_grid& g, const PBC& b, int i, i
     const T x00p = X(0, 0, 1), x00m = X(0, 0, -1);
     const T xp0p = X(1, 0, 1), xp0m = X(1, 0, -1), xm0p = X(-1, 0, 1), xm0m = X(-1, 0, -1);
     const T x0pp = X(0, 1, 1), x0pm = X(0, 1, -1), x0mp = X(0, -1, 1), x0mm = X(0, -1, -1);
-    const int sy = static_cast<int>(g.sy), sz = static_cast<int>(g.sz);
     T px_hi = (xp00 - x000) * dxinv;
     T pz_hi_md_hi = h * (xp0p + x00p - xp00 - x000);
-    pz_hi_md_hi *= m.rx[o + 1 + sz];
+    pz_hi_md_hi *= c.rxhh;
     T pz_hi_md_lo = h * (xp00 + x000 - xp0m - x00m);
-    pz_hi_md_lo *= m.rx[o + 1];
+    pz_hi_md_lo *= c.rxhl;
     px_hi -= h * (pz_hi_md_hi + pz_hi_md_lo);
 
     T px_lo = (x000 - xm00) * dxinv;
     T pz_lo_md_hi = h * (x00p + xm0p - x000 - xm00);
-    pz_lo_md_hi *= m.rx[o + sz];
+    pz_lo_md_hi *= c.rxlh;
     T pz_lo_md_lo = h * (x000 + xm00 - x00m - xm0m);
-    pz_lo_md_lo *= m.rx[o];
+    pz_lo_md_lo *= c.rxll;
     px_lo -= h * (pz_lo_md_hi + pz_lo_md_lo);
 
     T py_hi = (x0p0 - x000) * dyinv;
     T pz_md_hi_hi = h * (x0pp + x00p - x0p0 - x000);
-    pz_md_hi_hi *= m.ry[o + sy + sz];
+    pz_md_hi_hi *= c.ryhh;
     T pz_md_hi_lo = h * (x0p0 + x000 - x0pm - x00m);
-    pz_md_hi_lo *= m.ry[o + sy];
+    pz_md_hi_lo *= c.ryhl;
     py_hi -= h * (pz_md_hi_hi + pz_md_hi_lo);
 
     T py_lo = (x000 - x0m0) * dyinv;
     T pz_md_lo_hi = h * (x00p + x0mp - x000 - x0m0);
-    pz_md_lo_hi *= m.ry[o + sz];
+    pz_md_lo_hi *= c.rylh;
     T pz_md_lo_lo = h * (x000 + x0m0 - x00m - x0mm);
-    pz_md_lo_lo *= m.ry[o];
+    pz_md_lo_lo *= c.ryll;
     py_lo -= h * (pz_md_lo_hi + pz_md_lo_lo);
 
     T pz_hi = x00p - x000;
-    pz_hi *= m.hz[o + sz];
+    pz_hi *= c.hzh;
     const T px_hi_md_hi = h * (xp0p - x00p + xp00 - x000) * dxinv;
     const T px_lo_md_hi = h * (x00p - xm0p + x000 - xm00) * dxinv;
     const T py_md_hi_hi = h * (x0pp - x00p + x0p0 - x000) * dyinv;
     const T py_md_lo_hi = h * (x00p - x0mp + x000 - x0m0) * dyinv;
-    pz_hi -= h * m.sx[o + sz] * ((px_hi_md_hi + px_lo_md_hi) - (pz_hi_md_hi + pz_lo_md_hi));
-    pz_hi -= h * m.sy[o + sz] * ((py_md_hi_hi + py_md_lo_hi) - (pz_md_hi_hi + pz_md_lo_hi));
+    pz_hi -= h * c.sxh * ((px_hi_md_hi + px_lo_md_hi) - (pz_hi_md_hi + pz_lo_md_hi));
+    pz_hi -= h * c.syh * ((py_md_hi_hi + py_md_lo_hi) - (pz_md_hi_hi + pz_md_lo_hi));
 
     T pz_lo = x000 - x00m;
-    pz_lo *= m.hz[o];
+    pz_lo *= c.hzl;
     const T px_hi_md_lo = h * (xp00 - x000 + xp0m - x00m) * dxinv;
     const T px_lo_md_lo = h * (x000 - xm00 + x00m - xm0m) * dxinv;
     const T py_md_hi_lo = h * (x0p0 - x000 + x0pm - x00m) * dyinv;
     const T py_md_lo_lo = h * (x000 - x0m0 + x00m - x0mm) * dyinv;
-    pz_lo -= h * m.sx[o] * ((px_hi_md_lo + px_lo_md_lo) - (pz_hi_md_lo + pz_lo_md_lo));
-    pz_lo -= h * m.sy[o] * ((py_md_hi_lo + py_md_lo_lo) - (pz_md_hi_lo + pz_md_lo_lo));
+    pz_lo -= h * c.sxl * ((px_hi_md_lo + px_lo_md_lo) - (pz_hi_md_lo + pz_lo_md_lo));
+    pz_lo -= h * c.syl * ((py_md_hi_lo + py_md_lo_lo) - (pz_md_hi_lo + pz_md_lo_lo));
     if (MASKS) {
         if (k == 0) { pz_lo = T(0); }
         if ((b.zf & TP_XLO) && i == 0) { px_lo = T(0); }
@@ -222,15 +239,24 @@ __device__ __forceinline__ T adotx_body(const gb_grid& g, const PBC& b, int i, i
         if ((b.zf & TP_YHI) && j == g.ny - 1) { py_hi = T(0); }
         if ((b.zf & TP_ZHI) && k == g.nz - 1) { pz_hi = T(0); }
     }
-    const T y = (axa[o + 1] * px_hi - axa[o] * px_lo) * dxinv
-              + (aya[o + sy] * py_hi - aya[o] * py_lo) * dyinv
-              + (aza[o + sz] * pz_hi - aza[o] * pz_lo) * dzinv;
-    T v = y / Jc[o];
+    const T y = (c.axh * px_hi - c.axl * px_lo) * dxinv
+              + (c.ayh * py_hi - c.ayl * py_lo) * dyinv
+              + (c.azh * pz_hi - c.azl * pz_lo) * dzinv;
+    T v = y / c.J;
     if (MASKS && (b.zf & TP_DGROUND) && k == 0) {
         // a Dirichlet ground: the ground-face flux ERF's kernel leaves out (Source/Poisson.cpp:162-189)
-        v += aza[o] * ground_flux_dir<T>(g, i, j, X, m.zn) * dzinv / Jc[o];
+        v += c.azl * ground_flux_dir<T>(g, i, j, X, zn) * dzinv / c.J;
     }
     return v;
+}
+
+//! adotx_coefs with the coefficients read at flat index o.
+template <typename T, bool MASKS, typename XA>
+__device__ __forceinline__ T adotx_body(const gb_grid& g, const PBC& b, int i, int j, int k, int64_t o, XA&& X,
+                                        const T* __restrict__ axa, const T* __restrict__ aya, const T* __restrict__ aza,
+                                        const T* __restrict__ Jc, const MeshRatios<T>& m)
+{
+    return adotx_coefs<T, MASKS>(g, b, i, j, k, X, load_cell_coefs<T>(g, o, axa, aya, aza, Jc, m), m.zn);
 }
 
 //! The operator at (i, j, k) with the neighbours read directly (INTERIOR: all

@@ -236,6 +236,39 @@ def test_gpu_vcycle_tail_fp32_tracks_per_level_launches(ctx, per):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape,per", [((8, 8, 2), (True, True)), ((8, 8, 33), (False, False)),
+                                       ((8, 8, 64), (True, False)), ((8, 8, 65), (False, True)),
+                                       ((8, 8, 128), (True, True)), ((24, 24, 42), (False, False)),
+                                       ((24, 24, 43), (False, False)), ((8, 12, 64), (True, False))])
+def test_gpu_coarsest_level_a_cell_a_thread(ctx, precision, shape, per):
+    """The coarsest level with a thread for each cell (2 to 128 levels: one to
+    four a lane; up to 256 and up to 512 cells, odd extents; 3 x 3 x 43 is
+    over the limit, on the columns' kernel): a V-cycle equals the
+    launch-by-launch one to rounding (a thousand roundings of relaxed values:
+    1e-12 in FP64, 2e-4 in FP32)."""
+    import ablsteadyrans_b200 as gb
+    g, z, J, ax, ay, az, _ = smooth_terrain_case(*shape, *per, hill=150.0)
+    bc = (PERIODIC if per[0] else NEUMANN, PERIODIC if per[1] else NEUMANN, NEUMANN,
+          PERIODIC if per[0] else DIRICHLET, PERIODIC if per[1] else DIRICHLET, DIRICHLET)
+    r = g.np_zeros()
+    r[g.valid(0)] = np.random.default_rng(14).standard_normal(r[g.valid(0)].shape)
+    out = []
+    try:
+        for kernel in (0, 1):
+            ctx.tune(gb.TUNE_MG_COARSE_KERNEL, kernel)
+            dz, dJ, dax, day, daz = _gpu_case(g, z, J, ax, ay, az)
+            opts = gb.PoissonOptions.default(precision=precision, nu1=1, nu2=1, nu_coarse=8, max_levels=12, min_coarse=2)
+            ps = gb.PoissonSolver(ctx, g, dz, dJ, bc, opts)
+            ps.set_coeffs(dax, day, daz)
+            out.append(to_host(ps.vcycle(to_dev(r))))
+            ps.close()
+    finally:
+        ctx.tune(gb.TUNE_MG_COARSE_KERNEL, 0)
+    assert rel_err(out[0], out[1], g.valid(0)) < (1e-12 if precision == 0 else 2e-4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("per", [(True, False), (False, True)])
 def test_gpu_coarse_kernel_equals_per_relaxation_launches(ctx, precision, per):
     """The single-block coarsest-level kernel performs the per-relaxation
