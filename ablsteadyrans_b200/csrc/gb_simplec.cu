@@ -169,7 +169,7 @@ __global__ void k_sum_partials(const double* __restrict__ partial, int n, double
     }
 }
 
-//! The mean of f over one k-plane of box b per block (block k: level k),
+//! The mean of f over one k-plane of box b per block (block x: the level, y: the field),
 //! summed in a fixed order (Predictor.cpp:286-306: the horizontal mean of the
 //! other component's residual per level, every face once).
 //! One block per level (blockDim.x = kLevelThreads): each thread sums its
@@ -177,9 +177,17 @@ __global__ void k_sum_partials(const double* __restrict__ partial, int n, double
 //! fixed order), then the block reduces them in a fixed tree.
 constexpr int kLevelThreads = 1024;
 
-__global__ void __launch_bounds__(kLevelThreads) k_level_mean(gb_grid g, Box b, const double* __restrict__ f,
-                                                              double npts_level, double* __restrict__ mean)
+struct LevelMeans {   // per blockIdx.y: the box, the field, its points a level, the means
+    Box b[2];
+    const double* f[2];
+    double points[2];
+    double* mean[2];
+};
+
+__global__ void __launch_bounds__(kLevelThreads) k_level_mean(gb_grid g, const __grid_constant__ LevelMeans M)
 {
+    const Box b = M.b[blockIdx.y];
+    const double* __restrict__ f = M.f[blockIdx.y];
     __shared__ double red[kLevelThreads / 32];
     const int k = blockIdx.x;
     const int nx = b.hi[0] - b.lo[0] + 1, ny = b.hi[1] - b.lo[1] + 1;
@@ -199,7 +207,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_level_mean(gb_grid g, Box b, 
     if (threadIdx.x < 32) {
         double t = red[threadIdx.x];
         t = warp_sum(t);
-        if (threadIdx.x == 0) { mean[k] = t / npts_level; }
+        if (threadIdx.x == 0) { M.mean[blockIdx.y][k] = t / M.points[blockIdx.y]; }
     }
 }
 
@@ -351,7 +359,6 @@ struct SimplecWork {
     double* theta_ref;
     double* conv0;
     double* conv1;
-    double* dmask[3];   // each component's Dirichlet points (dirichlet_rows: they depend on the conditions alone)
     double* level_sum[2];
     double* partial;
     double* sums;
@@ -1882,15 +1889,219 @@ __device__ __forceinline__ double face_weight(int side, int i, int j, int k, con
     return weight_of(side, dif, tr, dxinv);
 }
 
+//! The seven coefficients of a point's row.
+struct Row7 {
+    double xm, xp, ym, yp, zm, zp, p;
+};
+
+//! The row at o as the seven arrays hold it.
+__device__ __forceinline__ Row7 load_row(const double* __restrict__ A, int64_t cs, int64_t o)
+{
+    return Row7{A[GB_COEF_XM * cs + o], A[GB_COEF_XP * cs + o], A[GB_COEF_YM * cs + o], A[GB_COEF_YP * cs + o],
+                A[GB_COEF_ZM * cs + o], A[GB_COEF_ZP * cs + o], A[GB_COEF_P * cs + o]};
+}
+
+//! A value as it stands: the compiler contracts nothing across (what follows
+//! rounds as it did when the value came from memory).
+__device__ __forceinline__ void pin(double& v) { asm("" : "+d"(v)); }
+
+//! A boundary face's fold of the rows at its edge (apply_to_implicit).
+enum RowFold { kRowFree = 0, kRowIdentity, kRowToOther, kRowMinus, kRowPlus, kRowZero };
+
+//! What follows the coefficients: the rows' additions and folds, then the
+//! system's diagonal, SIMPLEC denominator and right-hand side.
+struct RowTail {
+    int fold[3][2];          // per direction: the low and the high face's RowFold
+    int edge[3];             // the high edge's index
+    const double* dsdk;      // the Patankar diagonal of k, or null
+    const double* drag;      // the ground's wall rows (the drag plane), or null
+    const double* ustar;     // the first cells' k rows (with wall_k)
+    const double* d0;
+    int wall_k;              // 0 none, 1 Dirichlet rows, 2 added
+    // the system (null dt: rows alone)
+    const double* dt;
+    const double* R;
+    double* ap;
+    double* dd;
+    double* rhs;
+    double inv_cap, s_margin;  // w: the cap on its vertical relaxation (inv_cap 0: none)
+    double fs, relax;          // u, v: the rotation's coupling through the other component's residual
+    const double* mean;
+    const double* other;       // null: none
+    double gt;                 // w: the buoyancy's coupling through theta's rows
+    const double* theta_p;     // theta's diagonal coefficients, null: none
+    const double* theta;
+    const double* Rtheta;
+};
+
+//! Is (i, j, k) a Dirichlet point (its row is the identity)?
+__device__ __forceinline__ bool row_identity(const RowTail& a, int i, int j, int k)
+{
+    const int c[3] = {i, j, k};
+    bool id = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        id = id || (a.fold[d][0] == kRowIdentity && c[d] == 0) || (a.fold[d][1] == kRowIdentity && c[d] == a.edge[d]);
+    }
+    return id;
+}
+
+//! The row's additions and folds in the order of the launches that make them
+//! one by one (turb_patankar, turb_wall_rows, turb_wall_k_rows, k_fold_rows).
+template <int T>
+__device__ __forceinline__ void finish_row(const RowTail& a, const gb_grid& g, const double* __restrict__ J, double dzinv,
+                                           int i, int j, int k, int64_t o, Row7& r)
+{
+    if (a.dsdk) { r.p += a.dsdk[o]; }
+    if (a.drag && k == 0) {
+        r.p -= r.zm;
+        r.zm = 0;
+        if (T == XF) {
+            r.p += 0.5 * (a.drag[plane_at(g, i - 1, j)] + a.drag[plane_at(g, i, j)]) * dzinv / interp<CC, XF>(J, g, i, j, 0);
+        } else if (T == YF) {
+            r.p += 0.5 * (a.drag[plane_at(g, i, j - 1)] + a.drag[plane_at(g, i, j)]) * dzinv / interp<CC, YF>(J, g, i, j, 0);
+        }
+        if (a.wall_k) {
+            const int64_t pl = plane_at(g, i, j);
+            const double w = fmax(a.ustar[pl], 0.01) / a.d0[pl];
+            if (a.wall_k == 1) {
+                r = Row7{0, 0, 0, 0, 0, 0, w};
+            } else {
+                r.p += w;
+            }
+        }
+    }
+    auto fold = [&](int kind, bool here, double& ghost, double& opposite) {
+        if (!here || kind == kRowFree) { return; }
+        if (kind == kRowIdentity) {
+            r = Row7{0, 0, 0, 0, 0, 0, 1};
+            return;
+        }
+        const double ag = ghost;
+        ghost = 0;
+        if (kind == kRowToOther) {
+            opposite += ag;
+        } else if (kind != kRowZero) {
+            r.p += (kind == kRowMinus) ? -ag : ag;
+        }
+    };
+    fold(a.fold[0][0], i == 0, r.xm, r.xp);
+    fold(a.fold[0][1], i == a.edge[0], r.xp, r.xm);
+    fold(a.fold[1][0], j == 0, r.ym, r.yp);
+    fold(a.fold[1][1], j == a.edge[1], r.yp, r.ym);
+    fold(a.fold[2][0], k == 0, r.zm, r.zp);
+    fold(a.fold[2][1], k == a.edge[2], r.zp, r.zm);
+}
+
+//! A cell scalar's system at a point: a_P = 1/dtau + A_P, rhs = -R.
+__device__ __forceinline__ void scalar_system(const RowTail& a, int64_t o, const Row7& r)
+{
+    a.rhs[o] = -a.R[o];
+    a.ap[o] = 1.0 / a.dt[o] + r.p;
+}
+
+//! Component C's system at a point (Predictor.cpp's rows): a_P, d and rhs
+//! with w's cap, the rotation's coupling of u and v and w's with theta.
+template <int C>
+__device__ __forceinline__ void momentum_system(const RowTail& a, const gb_grid& g, const double* __restrict__ z, int i, int j,
+                                                int k, int64_t o, const Row7& r)
+{
+    const double keep = row_identity(a, i, j, k) ? 0.0 : 1.0;
+    const double dt = a.dt[o];
+    double p = keep / dt + r.p;
+    const double nb = r.xm + r.xp + r.ym + r.yp + r.zm + r.zp;
+    double d = keep * (p - nb);
+    pin(p);
+    pin(d);
+    double rhs = -a.R[o];
+    if (C == 2 && a.inv_cap > 0) {
+        double term = a.inv_cap * (r.zm + r.zp);
+        if (a.s_margin > 0) {
+            const double hx = 0.5 * (z[at(g, i + 1, j + 1, k)] + z[at(g, i + 1, j, k)] - z[at(g, i, j + 1, k)] - z[at(g, i, j, k)]) * (1.0 / g.dx);
+            const double hy = 0.5 * (z[at(g, i + 1, j + 1, k)] + z[at(g, i, j + 1, k)] - z[at(g, i + 1, j, k)] - z[at(g, i, j, k)]) * (1.0 / g.dy);
+            const double slope2 = hx * hx + hy * hy;
+            if (slope2 > 0) {
+                const double root = sqrt(1.0 + slope2) + 1.0;
+                const double rc = slope2 / (root * root);
+                const double lim = fmax(0.0, 1.0 / (a.s_margin * rc) - 1.0) / dt;
+                term = fmin(term, lim);
+            }
+        }
+        p += keep * term;
+        d += keep * term;
+        pin(p);
+        pin(d);
+    }
+    const int n = (C == 0) ? i : j;
+    if (C < 2 && a.other && keep != 0 && ((C == 0 ? g.periodic_x : g.periodic_y) || !(n == 0 || n == a.edge[C]))) {
+        const double fs = a.fs;
+        const double net = fmax(r.p - nb, 0.0);
+        const double tau_c = 1.0 / fmax(fabs(fs) / a.relax, net);
+        const double tau_own = 1.0 / (1.0 / dt + net);
+        const double stiff = fs * fs * fmax(tau_c, tau_own);
+        p += stiff;
+        d += stiff;
+        // four-face mean of the other component's residual with its periodic images resolved by index
+        auto RO = [&](int x, int y, int kk) {
+            const int nvx = g.nx + (C == 1 ? 1 : 0), nvy = g.ny + (C == 0 ? 1 : 0);
+            if (x < 0 || x >= nvx) {
+                if (!g.periodic_x) { return a.other[at(g, x, y, kk)]; }
+                x = (x < 0) ? x + g.nx : x - g.nx;
+            }
+            if (y < 0 || y >= nvy) {
+                if (!g.periodic_y) { return a.other[at(g, x, y, kk)]; }
+                y = (y < 0) ? y + g.ny : y - g.ny;
+            }
+            return a.other[at(g, x, y, kk)];
+        };
+        double avg;
+        if (C == 0) {  // interp<YF, XF>: v at (i-1..i, j..j+1)
+            avg = ((RO(i - 1, j, k) + RO(i, j, k)) + (RO(i - 1, j + 1, k) + RO(i, j + 1, k))) * 0.25;
+        } else {       // interp<XF, YF>: u at (i..i+1, j-1..j)
+            avg = ((RO(i, j - 1, k) + RO(i + 1, j - 1, k)) + (RO(i, j, k) + RO(i + 1, j, k))) * 0.25;
+        }
+        const double m = a.mean[k];
+        rhs += ((C == 0) ? -fs : fs) * (tau_c * m + tau_own * (avg - m));
+    }
+    if (C == 2 && a.theta_p && keep != 0) {
+        const double gt = a.gt;
+        auto zc = [&](int kk) {
+            return 0.125 * (z[at(g, i, j, kk)] + z[at(g, i + 1, j, kk)] + z[at(g, i, j + 1, kk)] + z[at(g, i + 1, j + 1, kk)]
+                            + z[at(g, i, j, kk + 1)] + z[at(g, i + 1, j, kk + 1)] + z[at(g, i, j + 1, kk + 1)]
+                            + z[at(g, i + 1, j + 1, kk + 1)]);
+        };
+        const int64_t om = at(g, i, j, k - 1);
+        const double gamma = (a.theta[o] - a.theta[om]) / (zc(k) - zc(k - 1));
+        const double ap_theta = 0.5 * (a.theta_p[om] + a.theta_p[o]);
+        const double tau = 1.0 / (1.0 / dt + ap_theta);
+        const double stiff = gt * fmax(gamma, 0.0) * tau;
+        p += stiff;
+        d += stiff;
+        rhs -= gt * tau * 0.5 * (a.Rtheta[om] + a.Rtheta[o]);
+    }
+    a.ap[o] = p;
+    a.dd[o] = d;
+    a.rhs[o] = rhs;
+}
+
+//! What a launch of k_fused_coefficients makes: the coefficients alone, the
+//! rows, the rows and the system, the rows' diagonal alone.
+enum RowMode { kCoefs = 0, kRows, kSystem, kDiagonal };
+
+
 //! The implicit coefficients with each face's parts evaluated once per block
 //! (the layout of k_fused_residual: 32 x 8 columns marching kc levels, the
-//! low x and y faces in shared memory, the z faces in registers).
-template <int C>
+//! low x and y faces in shared memory, the z faces in registers), and by MODE
+//! what follows them at the point (RowTail) while the row is in registers.
+//! Four blocks an SM whatever the mode: the launch is bound by latency (with
+//! the system at 128 x 128 x 64: 77 us at four, 86 at three, 118 at two, 78 at
+//! five with spills).
+template <int C, int MODE>
 __global__ void __launch_bounds__(kFusedTx* kFusedTy, 4)
     k_fused_coefficients(const gb_grid g, int ni, int nj, int nk, int kc, const double* __restrict__ z,
                          const double* __restrict__ J, int logz, const double* __restrict__ F0,
                          const double* __restrict__ F1, const double* __restrict__ F2, const double* __restrict__ gm,
-                         double* __restrict__ A)
+                         double* __restrict__ A, const __grid_constant__ RowTail tail)
 {
     pdl_entry();
     constexpr int T = (C < 0) ? CC : (1 << C);
@@ -1919,25 +2130,64 @@ __global__ void __launch_bounds__(kFusedTx* kFusedTy, 4)
         __syncthreads();
         if (active) {
             const double Jinv = 1.0 / interp<CC, T>(J, g, i, j, k);
-            const double xm = weight_of(0, xdif[ty][tx], xtr[ty][tx], dxinv) * Jinv;
-            const double xp = weight_of(1, xdif[ty][tx + 1], xtr[ty][tx + 1], dxinv) * Jinv;
-            const double ym = weight_of(0, ydif[ty][tx], ytr[ty][tx], dyinv) * Jinv;
-            const double yp = weight_of(1, ydif[ty + 1][tx], ytr[ty + 1][tx], dyinv) * Jinv;
-            const double zm = weight_of(0, zdif_lo, ztr_lo, dzinv) * Jinv;
-            const double zp = weight_of(1, zdif_hi, ztr_hi, dzinv) * Jinv;
+            Row7 r;
+            r.xm = weight_of(0, xdif[ty][tx], xtr[ty][tx], dxinv) * Jinv;
+            r.xp = weight_of(1, xdif[ty][tx + 1], xtr[ty][tx + 1], dxinv) * Jinv;
+            r.ym = weight_of(0, ydif[ty][tx], ytr[ty][tx], dyinv) * Jinv;
+            r.yp = weight_of(1, ydif[ty + 1][tx], ytr[ty + 1][tx], dyinv) * Jinv;
+            r.zm = weight_of(0, zdif_lo, ztr_lo, dzinv) * Jinv;
+            r.zp = weight_of(1, zdif_hi, ztr_hi, dzinv) * Jinv;
+            r.p = ((r.xm + r.xp) + (r.ym + r.yp)) + (r.zm + r.zp);
             const int64_t o = at(g, i, j, k);
-            A[GB_COEF_XM * cs + o] = xm;
-            A[GB_COEF_XP * cs + o] = xp;
-            A[GB_COEF_YM * cs + o] = ym;
-            A[GB_COEF_YP * cs + o] = yp;
-            A[GB_COEF_ZM * cs + o] = zm;
-            A[GB_COEF_ZP * cs + o] = zp;
-            A[GB_COEF_P * cs + o] = ((xm + xp) + (ym + yp)) + (zm + zp);
+            if (MODE != kCoefs) {
+                pin(r.xm);
+                pin(r.xp);
+                pin(r.ym);
+                pin(r.yp);
+                pin(r.zm);
+                pin(r.zp);
+                pin(r.p);
+                finish_row<T>(tail, g, J, dzinv, i, j, k, o, r);
+            }
+            if (MODE != kDiagonal) {
+                A[GB_COEF_XM * cs + o] = r.xm;
+                A[GB_COEF_XP * cs + o] = r.xp;
+                A[GB_COEF_YM * cs + o] = r.ym;
+                A[GB_COEF_YP * cs + o] = r.yp;
+                A[GB_COEF_ZM * cs + o] = r.zm;
+                A[GB_COEF_ZP * cs + o] = r.zp;
+            }
+            A[GB_COEF_P * cs + o] = r.p;
+            if (MODE == kSystem) {
+                if (C < 0) {
+                    scalar_system(tail, o, r);
+                } else {
+                    momentum_system<(C < 0) ? 0 : C>(tail, g, z, i, j, k, o, r);
+                }
+            }
         }
         zdif_lo = zdif_hi;
         ztr_lo = ztr_hi;
         __syncthreads();
     }
+}
+
+template <int C, int MODE>
+void launch_coefficients(gb_ctx* ctx, const gb_grid& g, const double* z, const double* J, int logz, double* const* F,
+                         const double* gm, double* A, const RowTail& tail)
+{
+    constexpr int T = (C < 0) ? CC : (1 << C);
+    const int knob = ctx->tune[GB_TUNE_RESIDUAL];
+    const int ni = g.nx + (T & 1), nj = g.ny + ((T >> 1) & 1), nk = g.nz + ((T >> 2) & 1);
+    const int kc = (knob >= 2) ? knob : kFusedLevels;
+    const dim3 block(kFusedTx, kFusedTy);
+    const dim3 grid((ni + kFusedTx - 1) / kFusedTx, (nj + kFusedTy - 1) / kFusedTy, (nk + kc - 1) / kc);
+    span_begin(ctx, GB_KERNEL_COEFS);
+    launch_pdl(ctx->tune[GB_TUNE_PDL] != 1, k_fused_coefficients<C, MODE>, grid, block, 0, ctx->stream, g, ni, nj, nk, kc,
+               z, J, logz, static_cast<const double*>(F[0]), static_cast<const double*>(F[1]),
+               static_cast<const double*>(F[2]), gm, A, tail);
+    span_end(ctx);
+    ++ctx->launches;
 }
 
 //! ImplicitOperator.cpp:39-74 coefficients<C> (C = -1: a cell scalar) on
@@ -1952,17 +2202,8 @@ void implicit_coefficients_on(gb_ctx* ctx, const gb_grid g, const double* z, con
     const double* F0 = F[0];
     const double* F1 = F[1];
     const double* F2 = F[2];
-    const int knob = ctx->tune[GB_TUNE_RESIDUAL];
-    if (knob != 1) {
-        const int ni = g.nx + (T & 1), nj = g.ny + ((T >> 1) & 1), nk = g.nz + ((T >> 2) & 1);
-        const int kc = (knob >= 2) ? knob : kFusedLevels;
-        const dim3 block(kFusedTx, kFusedTy);
-        const dim3 grid((ni + kFusedTx - 1) / kFusedTx, (nj + kFusedTy - 1) / kFusedTy, (nk + kc - 1) / kc);
-        span_begin(ctx, GB_KERNEL_COEFS);
-        launch_pdl(ctx->tune[GB_TUNE_PDL] != 1, k_fused_coefficients<C>, grid, block, 0, ctx->stream, g, ni, nj, nk,
-                   kc, z, J, logz, F0, F1, F2, gm, A);
-        span_end(ctx);
-        ++ctx->launches;
+    if (ctx->tune[GB_TUNE_RESIDUAL] != 1) {
+        launch_coefficients<C, kCoefs>(ctx, g, z, J, logz, F, gm, A, RowTail{});
         return;
     }
     for_box(ctx, valid_box(g, T), [=] __device__(int i, int j, int k) {
@@ -2114,12 +2355,69 @@ void dirichlet_rows(gb_simplec* S, int f, int t, double* mask)
 
 }  // namespace
 
+namespace {
+
+//! What follows equation eq's coefficients in its rows.
+RowTail row_tail(gb_simplec* S, int eq)
+{
+    const gb_grid& g = S->g;
+    const int t = (eq <= F_W) ? (1 << eq) : CC;
+    RowTail a{};
+    for (int d = 0; d < 3; ++d) {
+        const bool nod = nodal(t, d);
+        a.edge[d] = ((d == 0) ? g.nx : (d == 1) ? g.ny : g.nz) - (nod ? 0 : 1);
+        if (is_per(g, d)) { continue; }
+        for (int hi = 0; hi < 2; ++hi) {
+            const int rule = rule_for(eq, S->bc.face[d + 3 * hi], d, hi == 0);
+            a.fold[d][hi] = nod ? ((rule == R_VALUE || rule == R_PROFILE) ? kRowIdentity : kRowToOther)
+                          : (rule == R_EVEN) ? kRowMinus
+                          : (rule == R_ODD || rule == R_VALUE) ? kRowPlus
+                          : (rule == R_GRADIENT) ? kRowToOther : kRowZero;
+        }
+    }
+    if (S->ph.closure && eq == F_TKE) { a.dsdk = S->cf[kClosureDSdk]; }
+    if (S->wall && eq != F_W) {
+        a.drag = S->ss[kSsDrag];
+        if (eq == F_TKE) {
+            a.ustar = S->ss[kSsUstar];
+            a.d0 = S->ss[kSsD0];
+            a.wall_k = (S->bc.surface_wall_k == GB_WALL_K_DIRICHLET) ? 1 : 2;
+        }
+    }
+    return a;
+}
+
+//! The rows take one launch with their coefficients unless these are launched
+//! face by face (GB_TUNE_RESIDUAL = 1) or a damping layer adds to the diagonal.
+bool rows_fused(gb_simplec* S) { return S->ctx->tune[GB_TUNE_RESIDUAL] != 1 && !damping_of(S).on; }
+
+template <int MODE>
+void fused_rows(gb_simplec* S, int eq, double* const* F, double* A, const RowTail& a)
+{
+    gb_ctx* ctx = S->ctx;
+    const double *z = S->z, *J = S->mesh.detJ;
+    const int lz = S->ph.log_mean;
+    switch (eq) {
+    case F_U: launch_coefficients<0, MODE>(ctx, S->g, z, J, lz, F, S->dfe.nu, A, a); break;
+    case F_V: launch_coefficients<1, MODE>(ctx, S->g, z, J, lz, F, S->dfe.nu, A, a); break;
+    case F_W: launch_coefficients<2, MODE>(ctx, S->g, z, J, lz, F, S->dfe.nu, A, a); break;
+    case F_THETA: launch_coefficients<-1, MODE>(ctx, S->g, z, J, lz, F, S->dfe.gamma_theta, A, a); break;
+    default: launch_coefficients<-1, MODE>(ctx, S->g, z, J, lz, F, S->dfe.gamma_tke, A, a); break;
+    }
+}
+
+}  // namespace
+
 //! implicit_rows (Residual.cpp:272-304): the coefficients with the
 //! effective diffusivity, the Patankar diagonal of k with the closure, the
 //! first cells' wall rows (the surface state of the iteration's first fill)
 //! for every equation but w, then the boundary folds.
 void simplec_implicit_rows(gb_simplec* S, int eq, double* const* F, double* A)
 {
+    if (rows_fused(S)) {
+        fused_rows<kRows>(S, eq, F, A, row_tail(S, eq));
+        return;
+    }
     switch (eq) {
     case F_U: implicit_coefficients<0>(S, F, S->dfe.nu, A); break;
     case F_V: implicit_coefficients<1>(S, F, S->dfe.nu, A); break;
@@ -2134,6 +2432,31 @@ void simplec_implicit_rows(gb_simplec* S, int eq, double* const* F, double* A)
         if (eq == F_TKE) { turb_wall_k_rows(S->ctx, S->g, S->bc, S->ss, A); }
     }
     apply_to_implicit(S, eq, t, A);
+}
+
+//! Equation eq's rows into A and its system (a's arrays) at every point: one
+//! launch, the system's values taken from the rows in registers. Before, the
+//! coefficients' launch, up to four for the rows' additions and folds and one to
+//! two passes over the seven coefficients (u at 128 x 128 x 64: 53 + 4 + 12 +
+//! 19 + 30 us, now 77; k: 39 + 7 + 3 + 3 + 14 + 10, now 53).
+void implicit_system(gb_simplec* S, int eq, double* const* F, double* A, const RowTail& a)
+{
+    if (rows_fused(S)) {
+        fused_rows<kSystem>(S, eq, F, A, a);
+        return;
+    }
+    simplec_implicit_rows(S, eq, F, A);
+    const gb_grid g = S->g;
+    const int64_t cs = volume(g);
+    const double* z = S->z;
+    const int t = (eq <= F_W) ? (1 << eq) : CC;
+    for_box(S->ctx, valid_box(g, t), [=] __device__(int i, int j, int k) {
+        const int64_t o = at(g, i, j, k);
+        if (t == XF) { momentum_system<0>(a, g, z, i, j, k, o, load_row(A, cs, o)); }
+        else if (t == YF) { momentum_system<1>(a, g, z, i, j, k, o, load_row(A, cs, o)); }
+        else if (t == ZF) { momentum_system<2>(a, g, z, i, j, k, o, load_row(A, cs, o)); }
+        else { scalar_system(a, o, load_row(A, cs, o)); }
+    }, GB_KERNEL_COEFS);
 }
 
 // ------------------------------------------------------------ face dtau ---
@@ -2300,147 +2623,70 @@ gb_status momentum_predictor(gb_simplec* S, const gb_state& q, double** R, bool 
     const double fs = S->ph.coriolis ? 4 * 3.14159265358979323846 * std::sin(S->ph.latitude * 3.14159265358979323846 / 180)
                                          / S->ph.rotation_period
                                      : 0.0;
-    // each component's rows on a branch, theta's (the buoyancy coupling's) on a fourth
     const bool buoyant = S->ph.gravity > 0;
+    const bool rotates = S->ph.coriolis && fs != 0;
     Branches br(S);
     if (monitors) {
         br.on(4);
         residual_sums(S, q);
         dmax_velocity(S, q.u, q.v, q.w, W_MON_U);
     }
-    if (buoyant) {
-        br.on(3);
-        simplec_implicit_rows(S, F_THETA, w.F, w.At);
-    }
+    RowTail a[3];
     for (int c = 0; c < 3; ++c) {
-        br.on(c);
-        const int t = 1 << c;
-        simplec_implicit_rows(S, c, w.F, w.Am[c]);
-        double* ap = w.ap[c];
-        double* dd = w.dd[c];
-        const double* A = w.Am[c];
-        const double* mask = w.dmask[c];
-        const double* dt = w.dtf[c];
-        const double* Rc = R[c];
-        double* rhs = w.rhsm[c];
-        const double inv_cap = S->opt.w_vnn_cap > 0 ? 1.0 / S->opt.w_vnn_cap : 0.0;
-        const double s_margin = S->opt.w_vnn_cap_slope_margin;
-        const bool cap = (c == 2 && S->opt.w_vnn_cap > 0);
-        const double* z = S->z;
-        for_box(ctx, valid_box(g, t), [=] __device__(int i, int j, int k) {
-            const int64_t o = at(g, i, j, k);
-            const double keep = 1.0 - mask[o];
-            double p = keep / dt[o] + A[GB_COEF_P * cs + o];
-            const double nb = A[GB_COEF_XM * cs + o] + A[GB_COEF_XP * cs + o] + A[GB_COEF_YM * cs + o]
-                            + A[GB_COEF_YP * cs + o] + A[GB_COEF_ZM * cs + o] + A[GB_COEF_ZP * cs + o];
-            double d = keep * (p - nb);
-            if (cap) {
-                double term = inv_cap * (A[GB_COEF_ZM * cs + o] + A[GB_COEF_ZP * cs + o]);
-                if (s_margin > 0) {
-                    const double hx = 0.5 * (z[at(g, i + 1, j + 1, k)] + z[at(g, i + 1, j, k)] - z[at(g, i, j + 1, k)] - z[at(g, i, j, k)]) * (1.0 / g.dx);
-                    const double hy = 0.5 * (z[at(g, i + 1, j + 1, k)] + z[at(g, i, j + 1, k)] - z[at(g, i + 1, j, k)] - z[at(g, i, j, k)]) * (1.0 / g.dy);
-                    const double slope2 = hx * hx + hy * hy;
-                    if (slope2 > 0) {
-                        const double root = sqrt(1.0 + slope2) + 1.0;
-                        const double rc = slope2 / (root * root);
-                        const double lim = fmax(0.0, 1.0 / (s_margin * rc) - 1.0) / dt[o];
-                        term = fmin(term, lim);
-                    }
-                }
-                p += keep * term;
-                d += keep * term;
-            }
-            ap[o] = p;
-            dd[o] = d;
-            rhs[o] = -Rc[o];
-        }, GB_KERNEL_COEFS);
-        if (c < 2 && S->ph.coriolis && fs != 0) {
-            // the other component's residual: its horizontal mean per level
-            // (deterministic column-ordered sums), then the coupling
-            const double* other = (c == 0) ? R[1] : R[0];
-            const int to = (c == 0) ? YF : XF;
-            const int d_o = 1 - c;
-            const bool per_o = is_per(g, d_o);
-            const int n_o = (d_o == 0) ? g.nx : g.ny, n_c = (c == 0) ? g.nx : g.ny;
-            const double npts_level = static_cast<double>(n_o + (per_o ? 0 : 1)) * static_cast<double>(n_c);
-            {
-                // one block per level, a fixed summation order: deterministic
-                Box b = valid_box(g, to);
-                if (per_o) { b.hi[d_o] -= 1; }
-                Span span(ctx, GB_KERNEL_VECTOR);
-                k_level_mean<<<g.nz, kLevelThreads, 0, ctx->stream>>>(g, b, other, npts_level, w.level_sum[c]);
-                ++ctx->launches;
-            }
-            const double* mean = w.level_sum[c];
-            const double* og = other;  // read with its periodic images for the four-face mean
-            const bool px = g.periodic_x, py = g.periodic_y;
-            const double relax = S->opt.rotation_relax;
-            const bool per_c = is_per(g, c);
-            const int hi_edge = (c == 0) ? g.nx : g.ny;
-            const int cc = c;
-            for_box(ctx, valid_box(g, t), [=] __device__(int i, int j, int k) {
-                const int64_t o = at(g, i, j, k);
-                const double keep = 1.0 - mask[o];
-                if (keep == 0) { return; }
-                const int n = (cc == 0) ? i : j;
-                if (!per_c && (n == 0 || n == hi_edge)) { return; }
-                const double nb = A[GB_COEF_XM * cs + o] + A[GB_COEF_XP * cs + o] + A[GB_COEF_YM * cs + o]
-                                + A[GB_COEF_YP * cs + o] + A[GB_COEF_ZM * cs + o] + A[GB_COEF_ZP * cs + o];
-                const double net = fmax(A[GB_COEF_P * cs + o] - nb, 0.0);
-                const double tau_c = 1.0 / fmax(fabs(fs) / relax, net);
-                const double tau_own = 1.0 / (1.0 / dt[o] + net);
-                const double stiff = fs * fs * fmax(tau_c, tau_own);
-                ap[o] += stiff;
-                dd[o] += stiff;
-                // four-face mean with periodic images (og's ghosts resolved by index)
-                auto RO = [&](int a, int b2, int kk) {
-                    const int nvx = g.nx + (to & 1), nvy = g.ny + ((to >> 1) & 1);
-                    if (a < 0 || a >= nvx) {
-                        if (!px) { return og[at(g, a, b2, kk)]; }
-                        a = (a < 0) ? a + g.nx : a - g.nx;
-                    }
-                    if (b2 < 0 || b2 >= nvy) {
-                        if (!py) { return og[at(g, a, b2, kk)]; }
-                        b2 = (b2 < 0) ? b2 + g.ny : b2 - g.ny;
-                    }
-                    return og[at(g, a, b2, kk)];
-                };
-                double avg;
-                if (cc == 0) {  // interp<YF, XF>: v at (i-1..i, j..j+1)
-                    avg = ((RO(i - 1, j, k) + RO(i, j, k)) + (RO(i - 1, j + 1, k) + RO(i, j + 1, k))) * 0.25;
-                } else {        // interp<XF, YF>: u at (i..i+1, j-1..j)
-                    avg = ((RO(i, j - 1, k) + RO(i + 1, j - 1, k)) + (RO(i, j, k) + RO(i + 1, j, k))) * 0.25;
-                }
-                const double m = mean[k];
-                rhs[o] += ((cc == 0) ? -fs : fs) * (tau_c * m + tau_own * (avg - m));
-            }, GB_KERNEL_COEFS);
-        }
-        if (c == 2 && buoyant) {
-            br.join(2);
-            br.join(3);
-            const double gt = S->ph.gravity / S->ph.theta0;
-            const double* At = w.At;
-            const double* th = q.theta;
-            const double* Rt = R[4];
-            for_box(ctx, valid_box(g, ZF), [=] __device__(int i, int j, int k) {
-                const int64_t o = at(g, i, j, k);
-                const double keep = 1.0 - mask[o];
-                if (keep == 0) { return; }
-                auto zc = [&](int kk) {
-                    return 0.125 * (z[at(g, i, j, kk)] + z[at(g, i + 1, j, kk)] + z[at(g, i, j + 1, kk)] + z[at(g, i + 1, j + 1, kk)]
-                                    + z[at(g, i, j, kk + 1)] + z[at(g, i + 1, j, kk + 1)] + z[at(g, i, j + 1, kk + 1)]
-                                    + z[at(g, i + 1, j + 1, kk + 1)]);
-                };
-                const double gamma = (th[at(g, i, j, k)] - th[at(g, i, j, k - 1)]) / (zc(k) - zc(k - 1));
-                const double ap_theta = 0.5 * (At[GB_COEF_P * cs + at(g, i, j, k - 1)] + At[GB_COEF_P * cs + o]);
-                const double tau = 1.0 / (1.0 / dt[o] + ap_theta);
-                const double stiff = gt * fmax(gamma, 0.0) * tau;
-                ap[o] += stiff;
-                dd[o] += stiff;
-                rhs[o] -= gt * tau * 0.5 * (Rt[at(g, i, j, k - 1)] + Rt[o]);
-            }, GB_KERNEL_COEFS);
-        }
+        a[c] = row_tail(S, c);
+        a[c].dt = w.dtf[c];
+        a[c].R = R[c];
+        a[c].ap = w.ap[c];
+        a[c].dd = w.dd[c];
+        a[c].rhs = w.rhsm[c];
     }
+    if (S->opt.w_vnn_cap > 0) {
+        a[2].inv_cap = 1.0 / S->opt.w_vnn_cap;
+        a[2].s_margin = S->opt.w_vnn_cap_slope_margin;
+    }
+    if (buoyant) {
+        // theta's diagonal on w's branch, ahead of it
+        br.on(2);
+        if (rows_fused(S)) {
+            fused_rows<kDiagonal>(S, F_THETA, w.F, w.At, row_tail(S, F_THETA));
+        } else {
+            simplec_implicit_rows(S, F_THETA, w.F, w.At);
+        }
+        a[2].gt = S->ph.gravity / S->ph.theta0;
+        a[2].theta_p = w.At + GB_COEF_P * cs;
+        a[2].theta = q.theta;
+        a[2].Rtheta = R[4];
+    }
+    br.on(2);
+    implicit_system(S, F_W, w.F, w.Am[2], a[2]);
+    if (rotates) {
+        // each component's residual's horizontal mean per level, for the other's coupling
+        LevelMeans M{};
+        for (int c = 0; c < 2; ++c) {
+            const int o = 1 - c, to = 1 << o;
+            const int n_o = (o == 0) ? g.nx : g.ny, n_c = (c == 0) ? g.nx : g.ny;
+            M.b[c] = valid_box(g, to);
+            if (is_per(g, o)) { M.b[c].hi[o] -= 1; }
+            M.f[c] = R[o];
+            M.points[c] = static_cast<double>(n_o + (is_per(g, o) ? 0 : 1)) * static_cast<double>(n_c);
+            M.mean[c] = w.level_sum[c];
+            a[c].fs = fs;
+            a[c].relax = S->opt.rotation_relax;
+            a[c].mean = w.level_sum[c];
+            a[c].other = R[o];
+        }
+        br.on(1);
+        {
+            Span span(ctx, GB_KERNEL_VECTOR);
+            k_level_mean<<<dim3(g.nz, 2), kLevelThreads, 0, ctx->stream>>>(g, M);
+            ++ctx->launches;
+        }
+        br.join(1);
+    }
+    br.on(0);
+    implicit_system(S, F_U, w.F, w.Am[0], a[0]);
+    br.on(1);
+    implicit_system(S, F_V, w.F, w.Am[1], a[1]);
     br.join();
     // the three systems are independent: one batched solve
     const int locs[3] = {XF, YF, ZF};
@@ -2697,16 +2943,12 @@ gb_status scalar_sweeps(gb_simplec* S, const gb_state& q, const double* dtau, bo
     Branches br(S);
     for (int e = 0; e < 2; ++e) {
         br.on(e);
-        simplec_implicit_rows(S, eqs[e], w.F, w.Am[e]);
-        double* rhs = w.rhsm[e];
-        double* ap = w.ap[e];
-        const double* A = w.Am[e];
-        const double* Req = Rq[e];
-        for_box(ctx, valid_box(g, CC), [=] __device__(int i, int j, int k) {
-            const int64_t o = at(g, i, j, k);
-            rhs[o] = -Req[o];
-            ap[o] = 1.0 / dtau[o] + A[GB_COEF_P * cs + o];
-        }, GB_KERNEL_COEFS);
+        RowTail a = row_tail(S, eqs[e]);
+        a.dt = dtau;
+        a.R = Rq[e];
+        a.ap = w.ap[e];
+        a.rhs = w.rhsm[e];
+        implicit_system(S, eqs[e], w.F, w.Am[e], a);
     }
     br.join();
     const int locs[2] = {CC, CC};
@@ -2929,15 +3171,12 @@ gb_status simplec_scalar_step(gb_simplec* S, const gb_state& q, int eq, const do
     // the iteration refills them before the sweeps (Simplec.cpp:494-495)
     fill_ghosts_into(S, q, S->sst);
     transport_fluxes(S, q, w.F[0], w.F[1], w.F[2]);
-    simplec_implicit_rows(S, eq, w.F, w.Am[0]);
-    double* rhs = w.rhsm[0];
-    double* ap = w.ap[0];
-    const double* A = w.Am[0];
-    for_box(ctx, valid_box(g, CC), [=] __device__(int i, int j, int k) {
-        const int64_t o = at(g, i, j, k);
-        rhs[o] = -R_eq[o];
-        ap[o] = 1.0 / dtau[o] + A[GB_COEF_P * cs + o];
-    }, GB_KERNEL_COEFS);
+    RowTail a = row_tail(S, eq);
+    a.dt = dtau;
+    a.R = R_eq;
+    a.ap = w.ap[0];
+    a.rhs = w.rhsm[0];
+    implicit_system(S, eq, w.F, w.Am[0], a);
     const int word = (eq == F_THETA) ? W_LAST_TH : W_LAST_K;
     gb_status st = line_solve(S, CC, w.Am[0], w.ap[0], w.rhsm[0], w.deltam[0], word);
     if (st != GB_OK) { return st; }
@@ -3753,7 +3992,6 @@ gb_status simplec_build(gb_simplec* S)
     w.conv0 = dbuf(S, vol);
     w.conv1 = dbuf(S, vol);
     for (int n = 0; n < 2; ++n) { w.level_sum[n] = dbuf(S, g.nz + 1); }
-    for (int n = 0; n < 3; ++n) { w.dmask[n] = dbuf(S, vol); }
     w.partial = dbuf(S, static_cast<int64_t>(kRedBlocks) * (SUM_LEVEL + g.nz + 1));
     w.sums = dbuf(S, SUM_LEVEL + g.nz + 1);
     if (S->opt.precision == 1) {
@@ -3832,7 +4070,6 @@ gb_status simplec_build(gb_simplec* S)
         p.rt[n] = S->bc.theta_ref_theta[n];
     }
     if (S->ph.gravity > 0) { fill_theta_ref(S); }
-    for (int c = 0; c < 3; ++c) { dirichlet_rows(S, c, kLoc[c], w.dmask[c]); }
     // the Poisson solver of the correction (poisson_bc_from_faces, BoundaryConditions.cpp:362-380)
     int32_t pbc[6];
     for (int f = 0; f < 6; ++f) {

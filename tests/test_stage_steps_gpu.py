@@ -184,3 +184,62 @@ def test_gpu_parallel_branches_equal_one_stream(ctx, which, residual):
         ctx.tune(gb.TUNE_RESIDUAL, 0)
     for n, (a, b) in enumerate(zip(*out)):
         assert np.array_equal(a, b), n
+
+
+def _row_cases():
+    from test_simplec_gpu import CONFIGS, make, physics
+    for name in CONFIGS:
+        case, bc = make(name, nx=35, ny=10, nz=7, seed=9)
+        yield case, bc, physics(case, coriolis=1, latitude=40.0, geostrophic=1, ug=7.0, vg=-1.0)
+    from test_turbulence import _hill_case
+    yield _hill_case()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", range(4))
+@pytest.mark.parametrize("wall_k", [0, 1])
+def test_gpu_rows_in_one_launch_equal_the_separate_ones(ctx, which, wall_k):
+    """The rows with their folds, wall terms and system in the coefficients'
+    launch equal the separate launches (GB_TUNE_RESIDUAL = 1), at ragged sizes
+    and every kind of face: the five equations' rows, the predictor's a_P and
+    d, the predicted state and both scalars. The two evaluate the same
+    operations, contracted differently: 1e-13 of an array's largest value for
+    the rows (the largest a_P for d), 1e-10 after three line sweeps."""
+    import ablsteadyrans_b200 as gb
+    from ablsteadyrans_b200.simplec import DeviceCase, SimplecStage
+    out = []
+    try:
+        for residual in (0, 1):
+            case, bc, ph = list(_row_cases())[which]
+            bc.surface_wall_k = wall_k
+            opts = SimplecOptions.make(zline_sweeps=3, w_vnn_cap=16.0, tke_floor=1e-3)
+            oracle.fill_ghosts(case, bc, ph)
+            dc = DeviceCase.from_oracle(case)
+            st = SimplecStage(ctx, dc, bc, ph, opts)
+            st.fill_ghosts()
+            dt = st.local_dtau(2.0)
+            R = st.residual()
+            ctx.tune(gb.TUNE_RESIDUAL, residual)
+            rows = [st.implicit_rows(e).cpu().numpy() for e in (0, 1, 2, 4, 5)]
+            _, ap, d = st.momentum_predictor(R, dt, with_fields=True)
+            st.scalar_sweep(4, R[4], dt)
+            st.scalar_sweep(5, R[5], dt)
+            out.append((rows, [a.cpu().numpy() for a in ap], [a.cpu().numpy() for a in d],
+                        {f: dc.host(f) for f in FIELDS}))
+            st.close()
+            ctx.tune(gb.TUNE_RESIDUAL, 0)
+    finally:
+        ctx.tune(gb.TUNE_RESIDUAL, 0)
+    g = case.grid
+    for e, (a, b) in enumerate(zip(out[0][0], out[1][0])):
+        v = (slice(None),) + g.valid((1, 2, 4, 0, 0)[e])
+        assert np.abs(a[v] - b[v]).max() <= 1e-13 * np.abs(b[v]).max(), e
+    for c in range(3):
+        v = g.valid(LOCS[c])
+        scale = np.abs(out[1][1][c][v]).max()
+        assert np.abs(out[0][1][c][v] - out[1][1][c][v]).max() <= 1e-13 * scale, ("ap", c)
+        assert np.abs(out[0][2][c][v] - out[1][2][c][v]).max() <= 1e-13 * scale, ("d", c)
+    for n, f in enumerate(FIELDS):
+        v = g.valid(LOCS[n])
+        a, b = out[0][3][f][v], out[1][3][f][v]
+        assert np.abs(a - b).max() <= 1e-10 * max(np.abs(b).max(), 1e-300), f
