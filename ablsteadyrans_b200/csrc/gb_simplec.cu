@@ -1258,6 +1258,7 @@ constexpr int kFusedLevels = 2;
 //! faces take the wall stress (set_ground_fluxes, SurfaceLayer.cpp:418-450).
 struct StressArgs {
     gb_grid g;
+    FastDiv row;            // b's points along i (k_box's mapping of threads to points)
     Box b;                  // the union of the pairs' flux boxes
     Box pb[3];              // each pair's flux box
     double* G[3];           // each pair's flux array
@@ -1287,12 +1288,12 @@ __global__ void __launch_bounds__(256, 4) k_momentum_stress(const StressArgs a)
     constexpr int D1 = (L == CC) ? 1 : (L == (XF ^ YF)) ? 0 : (L == (XF ^ ZF)) ? 0 : 1;
     constexpr int NP = (L == CC) ? 3 : 2;
     const Box& b = a.b;
-    const int64_t n = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (n >= b.count()) { return; }
-    const int nx = b.hi[0] - b.lo[0] + 1, ny = b.hi[1] - b.lo[1] + 1;
-    const int i = b.lo[0] + static_cast<int>(n % nx);
-    const int j = b.lo[1] + static_cast<int>((n / nx) % ny);
-    const int k = b.lo[2] + static_cast<int>(n / (static_cast<int64_t>(nx) * ny));
+    const int n = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (n >= a.row.d * (b.hi[1] - b.lo[1] + 1)) { return; }
+    const int jj = a.row.quot(n);
+    const int i = b.lo[0] + n - jj * a.row.d, j = b.lo[1] + jj;
+    const int k = b.lo[2] + static_cast<int>(blockIdx.y + blockIdx.z * gridDim.y);
+    if (k > b.hi[2]) { return; }
     auto inside = [&](const Box& p) {
         return i >= p.lo[0] && i <= p.hi[0] && j >= p.lo[1] && j <= p.hi[1] && k >= p.lo[2] && k <= p.hi[2];
     };
@@ -1364,10 +1365,13 @@ void momentum_stress(gb_simplec* S, const gb_state& q, Branches& br)
         a.wall = S->wall ? 1 : 0;
         a.taux = S->ssr[kSsTauX];
         a.tauy = S->ssr[kSsTauY];
-        const int64_t n = a.b.count();
+        a.row = FastDiv(a.b.hi[0] - a.b.lo[0] + 1);
+        const int64_t plane = static_cast<int64_t>(a.row.d) * (a.b.hi[1] - a.b.lo[1] + 1);
+        const int planes = a.b.hi[2] - a.b.lo[2] + 1, py = std::min(planes, 65535);
         span_begin(S->ctx, GB_KERNEL_RESIDUAL);
-        launch_pdl(S->ctx->tune[GB_TUNE_PDL] != 1, k_momentum_stress<L>, dim3(static_cast<unsigned>((n + 255) / 256)),
-                   dim3(256), 0, S->ctx->stream, a);
+        launch_pdl(S->ctx->tune[GB_TUNE_PDL] != 1, k_momentum_stress<L>,
+                   dim3(static_cast<unsigned>((plane + 255) / 256), py, (planes + py - 1) / py), dim3(256), 0,
+                   S->ctx->stream, a);
         span_end(S->ctx);
         ++S->ctx->launches;
     };
@@ -1439,32 +1443,48 @@ __device__ __forceinline__ void fused_face(const FusedResidualArgs& a, int i, in
     gd = scalar_diff_face<D>(a.q, a.gamma, a.z, a.logz, a.g, i, j, k);
 }
 
+//! The faces past a block's last column: the first warp evaluates them for the
+//! eight rows of kEdgeLevels levels at once, a lane a face. With the last lane of
+//! each row's warp evaluating its own, every warp went through the x face twice
+//! a level (a level: 5.6 face evaluations a warp, now 4.3 at two levels a block).
+constexpr int kEdgeLevels = 4;
+static_assert(kEdgeLevels * kFusedTy == kFusedTx, "a lane a face");
+
 //! R = div(convective flux) - div(diffusive flux) (+ the pressure gradient
 //! for a velocity component; for k the bounded form's - k div(transport) and
 //! the sources), in the operation order of the separate launches
 //! (Residual.cpp:159-256).
-template <int E>
-__global__ void __launch_bounds__(kFusedTx* kFusedTy, 4) k_fused_residual(const FusedResidualArgs a)
+//! (Bound by its loads' latency: 45 % of issue slots, FP64 pipe 20 %, DRAM 15 % at
+//! 128 x 128 x 64; so BLOCKS an SM is five, 48 registers with a few spills, where
+//! there are blocks for several waves, and four, spill-free, below.)
+template <int E, int BLOCKS>
+__global__ void __launch_bounds__(kFusedTx* kFusedTy, BLOCKS) k_fused_residual(const FusedResidualArgs a)
 {
     pdl_entry();
     constexpr int T = (E < 3) ? (1 << E) : CC;
     constexpr int lx = flux_lo(T, 0), ly = flux_lo(T, 1), lz = flux_lo(T, 2);
-    __shared__ double xc[kFusedTy][kFusedTx + 1], xd[kFusedTy][kFusedTx + 1];
+    __shared__ double xc[kFusedTy][kFusedTx], xd[kFusedTy][kFusedTx];
     __shared__ double yc[kFusedTy + 1][kFusedTx], yd[kFusedTy + 1][kFusedTx];
+    __shared__ double ec[kEdgeLevels][kFusedTy], ed[kEdgeLevels][kFusedTy];
     const gb_grid& g = a.g;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int i = blockIdx.x * kFusedTx + tx, j = blockIdx.y * kFusedTy + ty;
     const bool active = i < a.ni && j < a.nj;
     const bool xhi = active && (tx == kFusedTx - 1 || i == a.ni - 1);
     const bool yhi = active && (ty == kFusedTy - 1 || j == a.nj - 1);
+    const int iend = min((static_cast<int>(blockIdx.x) + 1) * kFusedTx, a.ni) + lx;  // the block's last x face
     const int kb = blockIdx.z * a.kc, ke = min(kb + a.kc, a.nk);
     double zc_lo = 0, zd_lo = 0;
     if (active && kb < ke) { fused_face<E, 2>(a, i, j, kb + lz, zc_lo, zd_lo); }
     for (int k = kb; k < ke; ++k) {
         double zc_hi = 0, zd_hi = 0;
+        const int m = (k - kb) % kEdgeLevels;
+        if (ty == 0 && m == 0) {
+            const int je = blockIdx.y * kFusedTy + tx % kFusedTy, q = tx / kFusedTy;
+            if (je < a.nj && k + q < ke) { fused_face<E, 0>(a, iend, je, k + q, ec[q][tx % kFusedTy], ed[q][tx % kFusedTy]); }
+        }
         if (active) {
             fused_face<E, 0>(a, i + lx, j, k, xc[ty][tx], xd[ty][tx]);
-            if (xhi) { fused_face<E, 0>(a, i + lx + 1, j, k, xc[ty][tx + 1], xd[ty][tx + 1]); }
             fused_face<E, 1>(a, i, j + ly, k, yc[ty][tx], yd[ty][tx]);
             if (yhi) { fused_face<E, 1>(a, i, j + ly + 1, k, yc[ty + 1][tx], yd[ty + 1][tx]); }
             fused_face<E, 2>(a, i, j, k + lz + 1, zc_hi, zd_hi);
@@ -1473,7 +1493,8 @@ __global__ void __launch_bounds__(kFusedTx* kFusedTy, 4) k_fused_residual(const 
         if (active) {
             const int64_t o = at(g, i, j, k);
             const double Jt = interp<CC, T>(a.J, g, i, j, k);
-            double r = ((xc[ty][tx + 1] - xc[ty][tx]) * (1.0 / g.dx) + (yc[ty + 1][tx] - yc[ty][tx]) * (1.0 / g.dy)
+            const double xch = xhi ? ec[m][ty] : xc[ty][tx + 1], xdh = xhi ? ed[m][ty] : xd[ty][tx + 1];
+            double r = ((xch - xc[ty][tx]) * (1.0 / g.dx) + (yc[ty + 1][tx] - yc[ty][tx]) * (1.0 / g.dy)
                         + (zc_hi - zc_lo) * (1.0 / g.dzeta))
                      / Jt;
             if (E == 4) {
@@ -1483,7 +1504,7 @@ __global__ void __launch_bounds__(kFusedTx* kFusedTy, 4) k_fused_residual(const 
                                  + (interp<ZF, SZ>(a.F2, g, i, j, k + lz + 1) - interp<ZF, SZ>(a.F2, g, i, j, k + lz)) * (1.0 / g.dzeta);
                 r -= a.q[o] * div / Jt;
             }
-            r -= ((xd[ty][tx + 1] - xd[ty][tx]) * (1.0 / g.dx) + (yd[ty + 1][tx] - yd[ty][tx]) * (1.0 / g.dy)
+            r -= ((xdh - xd[ty][tx]) * (1.0 / g.dx) + (yd[ty + 1][tx] - yd[ty][tx]) * (1.0 / g.dy)
                   + (zd_hi - zd_lo) * (1.0 / g.dzeta))
                / Jt;
             if (E < 3) { r += pressure_gradient_at<(E < 3 ? E : 0)>(a.p, a.z, a.J, a.ax, a.ay, g, i, j, k); }
@@ -1543,7 +1564,11 @@ void fused_residual(gb_simplec* S, const gb_state& q, double* R)
     const dim3 block(kFusedTx, kFusedTy);
     const dim3 grid((a.ni + kFusedTx - 1) / kFusedTx, (a.nj + kFusedTy - 1) / kFusedTy, (a.nk + a.kc - 1) / a.kc);
     span_begin(S->ctx, GB_KERNEL_RESIDUAL);
-    launch_pdl(S->ctx->tune[GB_TUNE_PDL] != 1, k_fused_residual<E>, grid, block, 0, S->ctx->stream, a);
+    // five blocks an SM from two waves of four on (128 x 128 x 64, five equations: 387 us at four, 365 at
+    // five; an iteration of 32 x 32 x 48, below one wave: 799 us at four, 810 at five)
+    const bool many = static_cast<int64_t>(grid.x) * grid.y * grid.z > 8 * S->ctx->num_sms;
+    launch_pdl(S->ctx->tune[GB_TUNE_PDL] != 1, many ? k_fused_residual<E, 5> : k_fused_residual<E, 4>, grid, block, 0,
+               S->ctx->stream, a);
     span_end(S->ctx);
     ++S->ctx->launches;
 }

@@ -108,6 +108,32 @@ def test_gpu_fused_residual_matches_separate_launches(ctx, name, levels):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(161, 97, 33), (129, 72, 64), (33, 9, 5)])
+def test_gpu_fused_residual_over_many_blocks(ctx, shape):
+    """Grids of several waves of the fused residual's blocks (five an SM) and
+    one of a few, with one column, row or level past the blocks' sizes: equal
+    to the separate launches to 1e-13 of each residual's largest value."""
+    import ablsteadyrans_b200 as gb
+    from ablsteadyrans_b200.simplec import DeviceCase, SimplecStage
+    case, bc = make("inflow", *shape, seed=6)
+    ph = physics(case, limiter=LIMITER_VAN_ALBADA, log_mean=1, coriolis=1, latitude=45.0)
+    dc = DeviceCase.from_oracle(case)
+    st = SimplecStage(ctx, dc, bc, ph, SimplecOptions.make())
+    try:
+        st.fill_ghosts()
+        R0 = [r.cpu().numpy() for r in st.residual()]
+        ctx.tune(gb.TUNE_RESIDUAL, 1)
+        R1 = [r.cpu().numpy() for r in st.residual()]
+    finally:
+        ctx.tune(gb.TUNE_RESIDUAL, 0)
+        st.close()
+    for n, (a, b) in enumerate(zip(R0, R1)):
+        v = case.grid.valid(LOCS[n])
+        scale = max(np.abs(b[v]).max(), 1e-300)
+        assert np.abs(a[v] - b[v]).max() <= 1e-13 * scale, (FIELDS[n], np.abs(a[v] - b[v]).max(), scale)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("sweep", [(0, 0), (1, 1)], ids=["zjacobi", "lusgs-alternate"])
 @pytest.mark.parametrize("name", list(CONFIGS))
 def test_gpu_iterations_match_oracle(ctx, name, sweep):
