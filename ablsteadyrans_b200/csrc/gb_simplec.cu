@@ -246,6 +246,7 @@ __global__ void __launch_bounds__(256) k_maxabs(gb_grid g, Box b, const double* 
 constexpr int kMaxRed = 8;
 struct RedItem {
     Box b;
+    FastDiv nx, ny;   // the box's extents (a 64-bit division a point cost more than the sum)
     const double* f;
     const double* mul;
     int mode;   // sums: 0 squares, 1 values
@@ -266,14 +267,23 @@ __global__ void k_sumsq_partial_many(gb_grid g, const __grid_constant__ RedPack 
     __shared__ double red[8];
     double s = 0;
     const int64_t n_tot = b.count();
-    const int nx = b.hi[0] - b.lo[0] + 1, ny = b.hi[1] - b.lo[1] + 1;
-    for (int64_t n = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; n < n_tot;
-         n += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int i = b.lo[0] + static_cast<int>(n % nx);
-        const int j = b.lo[1] + static_cast<int>((n / nx) % ny);
-        const int k = b.lo[2] + static_cast<int>(n / (static_cast<int64_t>(nx) * ny));
-        const double v = f[at(g, i, j, k)];
-        s += (mode == 0) ? v * v : v;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    const int64_t n0 = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    if (n_tot < (int64_t(1) << 31)) {
+        const int64_t o0 = at(g, b.lo[0], b.lo[1], b.lo[2]);
+#pragma unroll 4
+        for (int64_t n = n0; n < n_tot; n += step) {
+            const int m = static_cast<int>(n), r = it.nx.quot(m), k = it.ny.quot(r);
+            const double v = f[o0 + (m - r * it.nx.d) + (r - k * it.ny.d) * g.sy + k * g.sz];
+            s += (mode == 0) ? v * v : v;
+        }
+    } else {
+        for (int64_t n = n0; n < n_tot; n += step) {
+            const int64_t r = n / it.nx.d;
+            const double v = f[at(g, b.lo[0] + static_cast<int>(n % it.nx.d), b.lo[1] + static_cast<int>(r % it.ny.d),
+                                  b.lo[2] + static_cast<int>(r / it.ny.d))];
+            s += (mode == 0) ? v * v : v;
+        }
     }
     s = warp_sum(s);
     if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = s; }
@@ -609,6 +619,8 @@ RedItem red_item(const Box& b, const double* f, const double* mul, int mode, int
 {
     RedItem it{};
     it.b = b;
+    it.nx = FastDiv(b.hi[0] - b.lo[0] + 1);
+    it.ny = FastDiv(b.hi[1] - b.lo[1] + 1);
     it.f = f;
     it.mul = mul;
     it.mode = mode;
@@ -660,37 +672,36 @@ void fill_periodic_all(gb_simplec* S, double* const* f, const int* t, int nf)
         P.t[n] = t[n];
     }
     P.n = nf;
+    // (a field a plane of the launch: its planes are the fields' levels)
     if (g.periodic_x) {
-        Box b{{0, 0, 0}, {2 * ng - 1, g.ny, g.nz}};
-        for_box(S->ctx, b, [=] __device__(int l2, int j, int k) {
+        Box b{{0, 0, 0}, {2 * ng - 1, g.ny, nf * (g.nz + 1) - 1}};
+        for_box(S->ctx, b, [=] __device__(int l2, int j, int nk) {
+            const int n = nk / (g.nz + 1), k = nk - n * (g.nz + 1);
             const int l = (l2 % ng) + 1;
             const bool hi = l2 >= ng;
-            for (int n = 0; n < P.n; ++n) {
-                const int t = P.t[n];
-                const int nvx = g.nx + (t & 1), nvy = g.ny + ((t >> 1) & 1), nvz = g.nz + ((t >> 2) & 1);
-                if (j >= nvy || k >= nvz) { continue; }
-                double* a = P.p[n];
-                if (!hi) { a[at(g, -l, j, k)] = a[at(g, g.nx - l, j, k)]; }
-                else { a[at(g, nvx - 1 + l, j, k)] = a[at(g, nvx - 1 + l - g.nx, j, k)]; }
-            }
+            const int t = P.t[n];
+            const int nvx = g.nx + (t & 1), nvy = g.ny + ((t >> 1) & 1), nvz = g.nz + ((t >> 2) & 1);
+            if (j >= nvy || k >= nvz) { return; }
+            double* a = P.p[n];
+            if (!hi) { a[at(g, -l, j, k)] = a[at(g, g.nx - l, j, k)]; }
+            else { a[at(g, nvx - 1 + l, j, k)] = a[at(g, nvx - 1 + l - g.nx, j, k)]; }
         }, GB_KERNEL_BC);
     }
     if (g.periodic_y) {
         const int ilo = g.periodic_x ? -ng : 0;
-        Box b{{ilo, 0, 0}, {g.nx + ng, 2 * ng - 1, g.nz}};
+        Box b{{ilo, 0, 0}, {g.nx + ng, 2 * ng - 1, nf * (g.nz + 1) - 1}};
         const bool px = g.periodic_x;
-        for_box(S->ctx, b, [=] __device__(int i, int l2, int k) {
+        for_box(S->ctx, b, [=] __device__(int i, int l2, int nk) {
+            const int n = nk / (g.nz + 1), k = nk - n * (g.nz + 1);
             const int l = (l2 % ng) + 1;
             const bool hi = l2 >= ng;
-            for (int n = 0; n < P.n; ++n) {
-                const int t = P.t[n];
-                const int nvx = g.nx + (t & 1), nvy = g.ny + ((t >> 1) & 1), nvz = g.nz + ((t >> 2) & 1);
-                const int ihi = px ? nvx - 1 + ng : nvx - 1;
-                if (i > ihi || k >= nvz) { continue; }
-                double* a = P.p[n];
-                if (!hi) { a[at(g, i, -l, k)] = a[at(g, i, g.ny - l, k)]; }
-                else { a[at(g, i, nvy - 1 + l, k)] = a[at(g, i, nvy - 1 + l - g.ny, k)]; }
-            }
+            const int t = P.t[n];
+            const int nvx = g.nx + (t & 1), nvy = g.ny + ((t >> 1) & 1), nvz = g.nz + ((t >> 2) & 1);
+            const int ihi = px ? nvx - 1 + ng : nvx - 1;
+            if (i > ihi || k >= nvz) { return; }
+            double* a = P.p[n];
+            if (!hi) { a[at(g, i, -l, k)] = a[at(g, i, g.ny - l, k)]; }
+            else { a[at(g, i, nvy - 1 + l, k)] = a[at(g, i, nvy - 1 + l - g.ny, k)]; }
         }, GB_KERNEL_BC);
     }
 }
@@ -917,27 +928,21 @@ void omega_from_w(gb_simplec* S, const double* u, const double* v, const double*
     }, GB_KERNEL_MASSFLUX);
 }
 
-//! velocity_divergence (MassFlux.cpp:129-136): Omega on the fly, then the face divergence.
-void velocity_divergence(gb_simplec* S, const double* u, const double* v, const double* w, double* div)
-{
-    const gb_grid g = S->g;
-    const double* z = S->z;
-    const double* ax = S->mesh.ax;
-    const double* ay = S->mesh.ay;
-    const double* az = S->mesh.az;
-    const double* J = S->mesh.detJ;
-    // a thread takes kDivLevels levels of a column: each z-face's Omega is
-    // evaluated once and serves the cells below and above it
-    constexpr int kDivLevels = 4;
-    const Box b{{0, 0, 0}, {g.nx - 1, g.ny - 1, (g.nz + kDivLevels - 1) / kDivLevels - 1}};
-    for_box(S->ctx, b, [=] __device__(int i, int j, int seg) {
+//! The face divergence of velocity at L levels of a column (velocity_divergence).
+template <int L>
+struct DivergenceCells {
+    gb_grid g;
+    const double *u, *v, *w, *z, *ax, *ay, *az, *J;
+    double* div;
+    __device__ __forceinline__ void operator()(int i, int j, int seg) const
+    {
         auto om = [&](int kk) {
             return w[at(g, i, j, kk)] - deriv<NODE, ZF, 0>(z, g, i, j, kk) * (1.0 / g.dx) * interp<XF, ZF>(u, g, i, j, kk)
                  - deriv<NODE, ZF, 1>(z, g, i, j, kk) * (1.0 / g.dy) * interp<YF, ZF>(v, g, i, j, kk);
         };
-        const int k0 = seg * kDivLevels;
+        const int k0 = seg * L;
         double om_lo = om(k0);
-        for (int q = 0; q < kDivLevels; ++q) {
+        for (int q = 0; q < L; ++q) {
             const int k = k0 + q;
             if (k >= g.nz) { break; }
             const double om_hi = om(k + 1);
@@ -947,7 +952,33 @@ void velocity_divergence(gb_simplec* S, const double* u, const double* v, const 
                    / J[o];
             om_lo = om_hi;
         }
-    }, GB_KERNEL_MASSFLUX);
+    }
+};
+
+//! velocity_divergence (MassFlux.cpp:129-136): Omega on the fly, then the face divergence.
+void velocity_divergence(gb_simplec* S, const double* u, const double* v, const double* w, double* div)
+{
+    const gb_grid g = S->g;
+    const double* z = S->z;
+    const double* ax = S->mesh.ax;
+    const double* ay = S->mesh.ay;
+    const double* az = S->mesh.az;
+    const double* J = S->mesh.detJ;
+    // a thread takes L levels of a column: each z-face's Omega is evaluated once
+    // and serves the cells below and above it. Four levels where they leave eight
+    // blocks an SM (128 x 128 x 64: 24 us, 29 with a cell a thread), else a cell a
+    // thread (32 x 32 x 48: 7.5 us, 13 with four levels, 12 blocks)
+    auto launch = [&](auto Lc) {
+        constexpr int L = decltype(Lc)::value;
+        const Box b{{0, 0, 0}, {g.nx - 1, g.ny - 1, (g.nz + L - 1) / L - 1}};
+        for_box(S->ctx, b, DivergenceCells<L>{g, u, v, w, z, ax, ay, az, J, div}, GB_KERNEL_MASSFLUX);
+    };
+    const int64_t threads = static_cast<int64_t>(g.nx) * g.ny * ((g.nz + 3) / 4);
+    if (threads >= static_cast<int64_t>(S->ctx->num_sms) * 1536) {
+        launch(std::integral_constant<int, 4>{});
+    } else {
+        launch(std::integral_constant<int, 1>{});
+    }
 }
 
 template <int D>
@@ -1760,40 +1791,69 @@ void add_damping_to_implicit(gb_simplec* S, int f, int t, double* A)
     }, GB_KERNEL_COEFS);
 }
 
+//! The Dirichlet faces' rows of the residual in one launch, blockIdx.y a face:
+//! each face writes its own component's points (they took a launch each,
+//! 5-8 us of latency).
+struct RowFaces {
+    int n;
+    int d[6], face[6], profile[6];
+    FastDiv len[6];            // the face plane's points along its first direction
+    int rows[6];               // ... and along its second
+    const double* q[3];
+    double* R[3];
+};
+
+__global__ void k_apply_rows(gb_grid g, const __grid_constant__ RowFaces P, const __grid_constant__ Profile prof,
+                             const double* __restrict__ z)
+{
+    pdl_entry();
+    const int f = blockIdx.y, d = P.d[f];
+    const int n = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (n >= P.len[f].d * P.rows[f]) { return; }
+    const int b = P.len[f].quot(n), a = n - b * P.len[f].d;
+    const int i = (d == 0) ? P.face[f] : a, j = (d == 0) ? a : (d == 1) ? P.face[f] : b, k = (d == 2) ? P.face[f] : b;
+    double V;
+    if (d < 2) {
+        V = P.profile[f] ? prof.value(d, height_above_ground(z, g, 1 << d, i, j, k)) : 0.0;
+    } else {
+        V = deriv<NODE, ZF, 0>(z, g, i, j, k) * (1.0 / g.dx) * interp<XF, ZF>(P.q[0], g, i, j, k)
+          + deriv<NODE, ZF, 1>(z, g, i, j, k) * (1.0 / g.dy) * interp<YF, ZF>(P.q[1], g, i, j, k);
+    }
+    const int64_t o = at(g, i, j, k);
+    P.R[d][o] = P.q[d][o] - V;
+}
+
 //! apply_rows (BoundaryConditions.cpp:801-852).
 void apply_rows(gb_simplec* S, const gb_state& q, double** R)
 {
     const gb_grid g = S->g;
-    const Profile prof = S->prof;
-    const double* z = S->z;
+    RowFaces P{};
     const double* qv[3] = {q.u, q.v, q.w};
+    int64_t most = 0;
     for (int d = 0; d < 3; ++d) {
+        P.q[d] = qv[d];
+        P.R[d] = R[d];
         if (is_per(g, d)) { continue; }
         for (int lo = 1; lo >= 0; --lo) {
             const int fc = d + (lo ? 0 : 3);
             if (!dirichlet_normal(S->bc, fc)) { continue; }
-            const bool is_profile = S->bc.face[fc] == GB_FACE_INFLOW;
-            const int t = 1 << d;
-            Box b = valid_box(g, t);
-            const int face = lo ? 0 : ((d == 0) ? g.nx : (d == 1) ? g.ny : g.nz);
-            b.lo[d] = b.hi[d] = face;
-            double* Rd = R[d];
-            const double* qd = qv[d];
-            const double* u = q.u;
-            const double* v = q.v;
-            const int dd = d;
-            for_box(S->ctx, b, [=] __device__(int i, int j, int k) {
-                double V;
-                if (dd < 2) {
-                    V = is_profile ? prof.value(dd, height_above_ground(z, g, 1 << dd, i, j, k)) : 0.0;
-                } else {
-                    V = deriv<NODE, ZF, 0>(z, g, i, j, k) * (1.0 / g.dx) * interp<XF, ZF>(u, g, i, j, k)
-                      + deriv<NODE, ZF, 1>(z, g, i, j, k) * (1.0 / g.dy) * interp<YF, ZF>(v, g, i, j, k);
-                }
-                Rd[at(g, i, j, k)] = qd[at(g, i, j, k)] - V;
-            }, GB_KERNEL_BC);
+            const Box b = valid_box(g, 1 << d);
+            const int e0 = (d == 0) ? 1 : 0, e1 = (d == 2) ? 1 : 2;
+            P.d[P.n] = d;
+            P.face[P.n] = lo ? 0 : ((d == 0) ? g.nx : (d == 1) ? g.ny : g.nz);
+            P.profile[P.n] = S->bc.face[fc] == GB_FACE_INFLOW;
+            P.len[P.n] = FastDiv(b.hi[e0] + 1);
+            P.rows[P.n] = b.hi[e1] + 1;
+            most = std::max(most, static_cast<int64_t>(b.hi[e0] + 1) * (b.hi[e1] + 1));
+            ++P.n;
         }
     }
+    if (P.n == 0) { return; }
+    span_begin(S->ctx, GB_KERNEL_BC);
+    launch_pdl(S->ctx->tune[GB_TUNE_PDL] != 1, k_apply_rows, dim3(static_cast<unsigned>((most + 255) / 256), P.n), dim3(256),
+               0, S->ctx->stream, g, P, S->prof, S->z);
+    span_end(S->ctx);
+    ++S->ctx->launches;
 }
 
 }  // namespace

@@ -310,6 +310,12 @@ void turb_closure(gb_ctx* ctx, const gb_grid& g, const gb_bc& bc, const gb_physi
         O.p[kClosureNu][o] = nu_mol + nt;
         O.p[kClosureGammaTheta][o] = alpha_mol + ratio * nt;
         O.p[kClosureGammaTke][o] = nu_mol + nt * inv_sigma;
+        // the four fields' vertical ghosts: copies of the first and last levels
+        for (int side = 0; side < 2; ++side) {
+            if (k != (side ? gg.nz - 1 : 0)) { continue; }
+            const int64_t og = side ? o + gg.sz : o - gg.sz;
+            for (int m = 0; m < 4; ++m) { O.p[m][og] = O.p[m][o]; }
+        }
         if (i >= 0 && i < gg.nx && j >= 0 && j < gg.ny) {
             const double Ps = nt * S2, Pb = -ratio * nt * N2;
             O.p[kClosureLength][o] = p.L;
@@ -320,7 +326,6 @@ void turb_closure(gb_ctx* ctx, const gb_grid& g, const gb_bc& bc, const gb_physi
             O.p[kClosureDSdk][o] = (p.eps + pos_part(-Pb)) / p.k;
         }
     }, GB_KERNEL_RESIDUAL);
-    copy_vertical_ghosts(ctx, g, cf, 4);
 }
 
 void turb_surface_state(gb_ctx* ctx, const gb_grid& g, const gb_bc& bc, const gb_physics& ph, const gb_state& q,
@@ -413,7 +418,6 @@ void turb_ground_gradients(gb_ctx* ctx, const gb_grid& g, const gb_bc& bc, const
                            const double* z0map, double* const* gg_out)
 {
     const gb_grid gg = g;
-    const double unset = DBL_MAX;
     const Stable sc = stable_of(bc);
     const double kappa = bc.kappa;
     const double qs = (bc.surface_stability == GB_SURFACE_HEAT_FLUX) ? bc.surface_heat_flux : 0.0;
@@ -421,13 +425,24 @@ void turb_ground_gradients(gb_ctx* ctx, const gb_grid& g, const gb_bc& bc, const
     const CPlanes11 S = cplanes(ss);
     Planes3 O{};
     for (int n = 0; n < 3; ++n) { O.p[n] = gg_out[n]; }
-    // the surface state's columns -1..nx, -1..ny; every other column unset
+    // One launch: each column evaluates the gradient of the column it takes it
+    // from. The surface state's columns are -1..nx, -1..ny; a column outside the
+    // domain that images a domain column across the periodic directions takes
+    // that one's (FillBoundary), and what is left (the second ghost column of a
+    // non-periodic direction) takes the nearest domain column's along it.
     for_box(ctx, Box{{-2, -2, 0}, {g.nx + 1, g.ny + 1, 0}}, [=] __device__(int i, int j, int) {
-        const int64_t p = plane_at(gg, i, j);
-        if (i < -1 || i > gg.nx || j < -1 || j > gg.ny) {
-            for (int n = 0; n < 3; ++n) { O.p[n][p] = unset; }
-            return;
+        auto wrap = [](int n, int len) { return ((n % len) + len) % len; };
+        int si = gg.periodic_x ? wrap(i, gg.nx) : i, sj = gg.periodic_y ? wrap(j, gg.ny) : j;
+        if (si < 0 || si >= gg.nx || sj < 0 || sj >= gg.ny) {
+            if (i >= -1 && i <= gg.nx && j >= -1 && j <= gg.ny) {
+                si = i;
+                sj = j;
+            } else {
+                si = min(max(si, 0), gg.nx - 1);
+                sj = min(max(sj, 0), gg.ny - 1);
+            }
         }
+        const int64_t p = plane_at(gg, si, sj), po = plane_at(gg, i, j);
         const double zeta = fmax(fmin(S.p[kSsD0][p] * S.p[kSsInvL][p], 100.0), -100.0);
         double phi_m, phi_h;
         most_phi(zeta, sc, phi_m, phi_h);
@@ -438,29 +453,9 @@ void turb_ground_gradients(gb_ctx* ctx, const gb_grid& g, const gb_bc& bc, const
         const double tsafe = tmag + DBL_MIN;
         const double dir_x = tx / tsafe, dir_y = ty / tsafe;
         const double us = S.p[kSsUstar][p];
-        O.p[0][p] = us / s * dir_x * phi_m;
-        O.p[1][p] = us / s * dir_y * phi_m;
-        O.p[2][p] = -qs / (us * s) * phi_h;
-    }, GB_KERNEL_BC);
-    // FillBoundary: a column outside the domain that images a domain column
-    // across the periodic directions takes its value
-    for_box(ctx, Box{{-2, -2, 0}, {g.nx + 1, g.ny + 1, 0}}, [=] __device__(int i, int j, int) {
-        if (i >= 0 && i < gg.nx && j >= 0 && j < gg.ny) { return; }
-        int si = i, sj = j;
-        if (gg.periodic_x) { si = ((i % gg.nx) + gg.nx) % gg.nx; }
-        if (gg.periodic_y) { sj = ((j % gg.ny) + gg.ny) % gg.ny; }
-        if (si >= 0 && si < gg.nx && sj >= 0 && sj < gg.ny) {
-            for (int n = 0; n < 3; ++n) { O.p[n][plane_at(gg, i, j)] = O.p[n][plane_at(gg, si, sj)]; }
-        }
-    }, GB_KERNEL_BC);
-    // what is left takes the nearest domain column along the non-periodic
-    // directions (the columns read are never unset themselves)
-    for_box(ctx, Box{{-2, -2, 0}, {g.nx + 1, g.ny + 1, 0}}, [=] __device__(int i, int j, int) {
-        const int64_t p = plane_at(gg, i, j);
-        if (O.p[0][p] != unset) { return; }
-        const int ic = gg.periodic_x ? i : min(max(i, 0), gg.nx - 1);
-        const int jc = gg.periodic_y ? j : min(max(j, 0), gg.ny - 1);
-        for (int n = 0; n < 3; ++n) { O.p[n][p] = O.p[n][plane_at(gg, ic, jc)]; }
+        O.p[0][po] = us / s * dir_x * phi_m;
+        O.p[1][po] = us / s * dir_y * phi_m;
+        O.p[2][po] = -qs / (us * s) * phi_h;
     }, GB_KERNEL_BC);
 }
 

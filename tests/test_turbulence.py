@@ -753,3 +753,33 @@ def test_gpu_qnse_wall_model_matches_oracle(ctx):
             assert np.abs(R[n][v] - R_ref[n][v]).max() <= 1e-10 * max(np.abs(R_ref[n][v]).max(), 1e-300), n
     finally:
         st.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("px,py", [(True, True), (True, False), (False, True), (False, False)])
+@pytest.mark.parametrize("shape", [(5, 4, 4), (18, 35, 6)])
+def test_gpu_wall_gradient_ghosts_every_lateral_condition(ctx, px, py, shape):
+    """The surface layer's ground fill with every mix of periodic and open
+    sides, corners and both ghost columns included: each column's wall
+    gradient is the one of the column it images or, past an open side, of the
+    nearest domain column; the closure's fields with their vertical ghosts.
+    1e-12 of a field's largest value: logarithms to an ulp each side, one
+    multiplication by a height."""
+    from ablsteadyrans_b200.abi import (BC, FACE_INFLOW, FACE_OUTFLOW, FACE_SLIP_WALL, FACE_SURFACE_LAYER, Physics,
+                                        SimplecOptions)
+    from ablsteadyrans_b200.simplec import DeviceCase, SimplecStage
+    from helpers import terrain_simplec_case
+    case = terrain_simplec_case(*shape, px, py, hill=30.0, seed=5)
+    case.q["tke"][...] = np.abs(case.q["tke"]) + 0.2
+    bc = BC.make((0 if px else FACE_INFLOW, 0 if py else FACE_SLIP_WALL, FACE_SURFACE_LAYER, 0 if px else FACE_OUTFLOW,
+                  0 if py else FACE_SLIP_WALL, FACE_SLIP_WALL), theta_ref=((0.0, 1500.0), (300.0, 300.0)), ustar=0.4,
+                 z0=0.1, surface={"z0": 0.1})
+    ph = Physics.make(1500.0, closure=1, log_mean=1)
+    dc = DeviceCase.from_oracle(case)
+    st = SimplecStage(ctx, dc, bc, ph, SimplecOptions.make())
+    oracle.fill_ghosts(case, bc, ph)
+    st.fill_ghosts()
+    for f in FIELDS:
+        ref, got = case.q[f], dc.host(f)
+        assert np.abs(got - ref).max() <= 1e-12 * max(np.abs(ref).max(), 1.0), f
+    st.close()
