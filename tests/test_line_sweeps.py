@@ -203,6 +203,26 @@ def test_gpu_zline_jacobi_batch_equals_single_systems(ctx, segment, sweeps):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("sweeps", [1, 2])
+def test_gpu_zline_jacobi_batch_clears_ghosts_and_words(ctx, sweeps):
+    """The one launch that clears a batch's ghosts: increments that held NaN
+    come back with every point outside the valid ones 0 and the valid ones,
+    and the changes, those of a first call (uneven grids, every location)."""
+    import torch
+    gb, systems, _ = _batch_case(torch.float64, 0, 700)
+    want = gb.zline_jacobi_batch(ctx, systems, sweeps)
+    first = [s[5].clone() for s in systems]
+    for s in systems:
+        s[5].fill_(float("nan"))
+    assert gb.zline_jacobi_batch(ctx, systems, sweeps) == want
+    for a, (g, loc, *_, dd) in zip(first, systems):
+        assert torch.equal(a, dd), (g.nx, g.ny, g.nz, loc)
+        inside = torch.zeros_like(dd, dtype=torch.bool)
+        inside[g.valid(loc)] = True
+        assert bool((dd[~inside] == 0).all()), (g.nx, g.ny, g.nz, loc)
+
+
+@pytest.mark.gpu
 def test_gpu_zline_jacobi_batch_repeat_and_refusals(ctx):
     """A second batched call on the same context (the scratch and work-list
     reused) gives the same values; a system whose columns are taller than
