@@ -619,8 +619,8 @@ RedItem red_item(const Box& b, const double* f, const double* mul, int mode, int
 {
     RedItem it{};
     it.b = b;
-    it.nx = FastDiv(b.hi[0] - b.lo[0] + 1);
-    it.ny = FastDiv(b.hi[1] - b.lo[1] + 1);
+    it.nx = FastDiv(std::max(b.hi[0] - b.lo[0] + 1, 1));
+    it.ny = FastDiv(std::max(b.hi[1] - b.lo[1] + 1, 1));
     it.f = f;
     it.mul = mul;
     it.mode = mode;
@@ -1304,10 +1304,12 @@ struct StressArgs {
     const double* tauy;
 };
 
-//! (Four 256-thread blocks an SM, at most 64 registers a thread, as the fused
-//! residual and coefficient launches: each is bound by its loads' latency,
-//! and the fourth block's warps cut the residual evaluation's time by 12 %
-//! against three blocks at 72-84 registers, a few bytes of spills included.)
+//! (Four 256-thread blocks an SM, at most 64 registers a thread, as the
+//! coefficient launches: each is bound by its loads' latency, and the fourth
+//! block's warps cut the residual evaluation's time by 12 % against three
+//! blocks at 72-84 registers, a few bytes of spills included; five gain 10 %
+//! on two of the four launches and lose 7 % on one. Points by k_box's mapping:
+//! 128 x 128 x 64, the four: 135 us with 64-bit divisions, 125 so.)
 template <int L>
 __global__ void __launch_bounds__(256, 4) k_momentum_stress(const StressArgs a)
 {
