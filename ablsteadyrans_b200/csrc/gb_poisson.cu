@@ -1787,10 +1787,10 @@ __global__ void k_convert_all(T* __restrict__ dst, const double* __restrict__ sr
 // iterates do not depend on how many launches a step takes.
 
 //! Krylov vectors as a kernel argument: at one stride (N = 0: those that a
-//! solver makes with itself, which most solves stop within), or up to N by
-//! address (they are made as a solve needs them). Addresses cost the passes: 1.5
-//! to 4 % of a whole projection (152 x 88 x 57, 17 steps), as a launch copies
-//! its parameters and every vector's address is a load.
+//! solver makes with itself), or up to N by address (a borrowing solver's,
+//! which come from several places). Addresses cost the passes: 1.5 to 4 % of a
+//! whole projection (152 x 88 x 57, 17 steps), as a launch copies its parameters
+//! and every vector's address is a load.
 template <int N>
 struct Columns {
     const double* p[N];
@@ -2672,7 +2672,9 @@ bool strided(const std::vector<double*>& c, int n, Columns<0>& r)
     return true;
 }
 
-//! n steps' Krylov vectors: Z of each, V of each and the one after.
+//! n steps' Krylov vectors: Z of each, V of each and the one after. A solver
+//! with arrays of its own has them all; a borrowing one takes those past the
+//! lender's from `spare`, then allocates.
 gb_status ensure_columns(gb_poisson* P, int n)
 {
     const int64_t vol = (volume(P->g) + 31) / 32 * 32;
@@ -2898,14 +2900,12 @@ gb_status poisson_build(gb_poisson* P, gb_poisson* lender)
             }
         }
     }
-    // Krylov workspace. The vectors of the first steps come with it: as many of
-    // the restart's as kKrylovBytes hold (8 at least); further ones when a solve
-    // gets that far. All of them (restart 50: 101 volumes) were 5.5 GB on a
-    // 256 x 256 x 96 grid whose solves take 8 to 20 steps.
-    constexpr int64_t kKrylovBytes = int64_t(512) << 20;
+    // Krylov workspace: all of the restart's vectors, so that a solve allocates
+    // nothing. (Making them as steps need them saved most of the 5.5 GB of a
+    // restart of 50 on 256 x 256 x 96, but then a solve could fail for memory
+    // half-way, and its cudaMalloc broke other threads' stream captures.)
     const int64_t vol = volume(P->g), vs = (vol + 31) / 32 * 32;
     const int m = P->opt.restart;
-    const int pairs = static_cast<int>(std::min<int64_t>(m, std::max<int64_t>(kKrylovChunk, kKrylovBytes / (16 * vs))));
     P->dot_blocks = std::min(4 * ctx->num_sms, nblocks(static_cast<int64_t>(P->g.nx) * P->g.ny * P->g.nz));
     if (lender != nullptr) {
         P->w = lender->w;
@@ -2926,8 +2926,8 @@ gb_status poisson_build(gb_poisson* P, gb_poisson* lender)
             P->t = a.take<double>(vol);
             P->Vc.clear();
             P->Zc.clear();
-            for (int q = 0; q <= pairs; ++q) { P->Vc.push_back(a.take<double>(vs)); }
-            for (int q = 0; q < pairs; ++q) { P->Zc.push_back(a.take<double>(vs)); }
+            for (int q = 0; q <= m; ++q) { P->Vc.push_back(a.take<double>(vs)); }
+            for (int q = 0; q < m; ++q) { P->Zc.push_back(a.take<double>(vs)); }
         }
     });
     if (!ok) {

@@ -59,8 +59,9 @@ struct gb_poisson {
     double* cross_store[2]{nullptr, nullptr};
     // Krylov workspace
     // The basis and the preconditioned vectors, one padded volume each (their
-    // ghosts are never read): made as the steps of a solve need them, from
-    // `spare` volumes first (a lender's), then in chunks of kKrylovChunk pairs.
+    // ghosts are never read): all made with the solver. A borrowing one starts
+    // with the lender's and takes further ones as the steps of a solve need
+    // them, from `spare` volumes first, then in chunks of kKrylovChunk pairs.
     std::vector<double*> Vc, Zc;
     std::vector<double*> spare;
     std::vector<void*> chunks;

@@ -297,7 +297,9 @@ gb_status gb_poisson_options_default(gb_poisson_opts* opt);
 
 /* gust::PoissonSolver (Source/Poisson.H:135-161) for the mesh (z_nd, detJ:
  * device arrays kept by reference, as the reference's solver keeps the mesh)
- * and the boundary types bc[6]. Builds the multigrid hierarchy. */
+ * and the boundary types bc[6]. Builds the multigrid hierarchy and allocates the
+ * restart's Krylov vectors (2 restart + 1 arrays of the grid): gb_poisson_solve
+ * allocates none. */
 gb_status gb_poisson_create(gb_ctx* ctx, const gb_grid* g, const int32_t* bc, const double* z_nd, const double* detJ,
                             const gb_poisson_opts* opt, gb_poisson** out);
 gb_status gb_poisson_destroy(gb_poisson* p);
@@ -678,7 +680,9 @@ gb_status gb_init_options_default(gb_init_opts* o);
  * solve with lambda = 0 on the inflow and outflow faces and zero flux through
  * the others, Sigma = diag(alpha_h^2, alpha_h^2, alpha_v^2) with the split
  * z-face coefficient when alpha_v != alpha_h (u, v, Omega += the fluxes, w
- * from Omega). */
+ * from Omega). The projection may allocate device memory while it runs (a solver
+ * where the stage's own cannot lend its arrays, vectors past those the stage
+ * holds) and gives it back before the call returns. */
 gb_status gb_simplec_initialize(gb_simplec* s, const gb_state* q, const gb_init_opts* o, gb_init_result* r);
 
 /* What a prolongation did (gust::ProlongResult, Source/Transfer.H:112-116). */

@@ -571,3 +571,32 @@ def test_gpu_one_launch_colours_give_the_two_launch_vcycle(ctx, case, precision)
     if precision == 0:
         mg = oracle.Multigrid(g, bc, z, J, ax, ay, az, max_levels=12, min_coarse=2, nu1=1, nu2=1, nu_coarse=8)
         assert rel_err(out[0], mg.vcycle(r), v) < 1e-12
+
+
+@pytest.mark.gpu
+def test_gpu_solve_takes_no_device_memory(ctx):
+    """A solver holds all of its restart's vectors from its creation on: a
+    solve that uses every one of them (48 steps of a single level's
+    relaxation, which do not converge; 97 vectors of 7 MB, 690 MB) leaves the
+    device's free memory where a solve of two steps left it."""
+    import torch
+
+    import ablsteadyrans_b200 as gb
+    g, z, J, ax, ay, az, _ = smooth_terrain_case(128, 112, 56, False, False, hill=150.0)
+    bc = (NEUMANN, NEUMANN, NEUMANN, DIRICHLET, NEUMANN, NEUMANN)
+    rhs = g.np_zeros()
+    v = g.valid(0)
+    rhs[v] = np.random.default_rng(8).standard_normal(rhs[v].shape)
+    dz, dJ, dax, day, daz = _gpu_case(g, z, J, ax, ay, az)
+    free = []
+    for max_iter in (2, 48):
+        opts = gb.PoissonOptions.default(reltol=1e-12, restart=48, max_iter=max_iter, max_levels=1, nu_coarse=1)
+        ps = gb.PoissonSolver(ctx, g, dz, dJ, bc, opts)
+        ps.set_coeffs(dax, day, daz)
+        drhs, phi = to_dev(rhs), to_dev(g.np_zeros())
+        before = torch.cuda.mem_get_info()[0]
+        with pytest.raises(gb.GustError, match="did not converge"):
+            ps.solve(drhs, phi)
+        free.append(before - torch.cuda.mem_get_info()[0])
+        ps.close()
+    assert free[1] - free[0] < 8 * g.volume, free
