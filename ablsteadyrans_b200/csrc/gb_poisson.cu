@@ -3225,8 +3225,10 @@ gb_status poisson_solve(gb_poisson* P, double* rhs, double* phi, gb_poisson_resu
         ++ctx->launches;
         last = -1.0;
     }
-    if (last < 0) {
-        // phi changed since its residual was last taken
+    if (last < 0 || it == 0) {
+        // phi changed since its residual was last taken, or no step applied the
+        // operator: a solve whose coefficients are not finite is refused
+        // whatever its right-hand side
         apply_fine(P, phi, rhs, P->w);
         double r2 = 0;
         if ((st = dot_host(P, P->w, P->w, &r2)) != GB_OK) { return st; }

@@ -600,3 +600,23 @@ def test_gpu_solve_takes_no_device_memory(ctx):
         free.append(before - torch.cuda.mem_get_info()[0])
         ps.close()
     assert free[1] - free[0] < 8 * g.volume, free
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("value", [0.0, 1.0])
+def test_gpu_solve_refuses_coefficients_that_are_not_finite(ctx, bad, value):
+    """One coefficient that is not finite: the solve is refused, also where
+    the right-hand side is zero and no step is taken."""
+    import ablsteadyrans_b200 as gb
+    g, z, J, ax, ay, az, _ = smooth_terrain_case(16, 12, 8, False, False, hill=30.0)
+    bc = (NEUMANN, NEUMANN, NEUMANN, DIRICHLET, NEUMANN, NEUMANN)
+    ax[g.ng + 3, g.ng + 4, g.ng + 5] = bad
+    dz, dJ, dax, day, daz = _gpu_case(g, z, J, ax, ay, az)
+    ps = gb.PoissonSolver(ctx, g, dz, dJ, bc, gb.PoissonOptions.default())
+    ps.set_coeffs(dax, day, daz)
+    rhs = g.np_zeros()
+    rhs[g.valid(0)] = value
+    with pytest.raises(gb.GustError, match="non-finite"):
+        ps.solve(to_dev(rhs), to_dev(g.np_zeros()))
+    ps.close()
