@@ -2052,19 +2052,8 @@ void gb_poisson::release_chunks()
 {
     if (chunks.empty()) { return; }
     cudaStreamSynchronize(ctx->stream);
-    // the vectors in the chunks leave the lists; the others stay
-    const int64_t vol = (gb::volume(g) + 31) / 32 * 32;
-    auto ours = [&](const double* p) {
-        for (void* c : chunks) {
-            const double* b = static_cast<const double*>(c);
-            if (p >= b && p < b + vol * 2 * gb::kKrylovChunk) { return true; }
-        }
-        return false;
-    };
-    for (auto* list : {&Vc, &Zc, &spare}) {
-        list->erase(std::remove_if(list->begin(), list->end(), ours), list->end());
-    }
-    for (void* c : chunks) { cudaFree(c); }
+    for (auto* list : {&Vc, &Zc, &spare}) { gb::forget_chunks(chunks, *list); }
+    for (const gb::KrylovChunk& c : chunks) { cudaFree(c.base); }
     chunks.clear();
 }
 
@@ -2687,7 +2676,7 @@ gb_status ensure_columns(gb_poisson* P, int n)
                 set_error("gust: PoissonSolver: cannot allocate the Krylov workspace");
                 return GB_OOM;
             }
-            P->chunks.push_back(p);
+            P->chunks.push_back(KrylovChunk{static_cast<double*>(p), vol * 2 * pairs});
             for (int q = 0; q < 2 * pairs; ++q) { P->spare.push_back(static_cast<double*>(p) + vol * q); }
         }
         auto& to = P->Vc.size() <= P->Zc.size() ? P->Vc : P->Zc;

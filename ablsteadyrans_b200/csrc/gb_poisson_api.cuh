@@ -1,6 +1,7 @@
 // Host-side state of the Poisson layer (the C ABI's gb_poisson handle).
 #pragma once
 
+#include "gb_krylov.h"
 #include "gb_poisson.cuh"
 
 #include <vector>
@@ -64,7 +65,7 @@ struct gb_poisson {
     // them, from `spare` volumes first, then in chunks of kKrylovChunk pairs.
     std::vector<double*> Vc, Zc;
     std::vector<double*> spare;
-    std::vector<void*> chunks;
+    std::vector<gb::KrylovChunk> chunks;
     unsigned long long* d_err{nullptr};    // set when a TMA tile wait gave up
     double* w{nullptr};
     double* t{nullptr};

@@ -419,3 +419,37 @@ def test_gpu_initializer_shares_the_correction_solvers_arrays(ctx, precision, re
         for n, (a, b) in enumerate(zip(got, want)):
             assert np.array_equal(a, b), n
     used.close()
+
+
+@pytest.mark.gpu
+def test_gpu_initializer_with_vectors_beyond_the_stages(ctx):
+    """An initial state whose projection takes more vectors than the stage's
+    arrays hold (16 steps' of a restart of 26: a full chunk and a short one
+    are made and given back), then again: the bits of the first one and of a
+    new stage's."""
+    from ablsteadyrans_b200 import abi, workloads
+    from ablsteadyrans_b200.simplec import FIELDS, DeviceCase, SimplecStage
+
+    def stage():
+        inst = workloads.tile(40, 24, 3)
+        inst.options.poisson.restart = 2
+        J, ax, ay, az, _ = oracle.metrics(inst.grid, inst.z)
+        dc = DeviceCase(inst.grid, inst.z, J, ax, ay, az, inst.nu, inst.gamma_theta, inst.gamma_tke, inst.q, inst.z0map)
+        return SimplecStage(ctx, dc, inst.bc, inst.physics, inst.options), dc
+
+    # (the split coefficients and a weak smoother: a slow solve on the levels of the stage's solver)
+    o = abi.InitOptions.make(alpha_v=0.3)
+    o.poisson.nu1, o.poisson.nu2, o.poisson.nu_coarse = 0, 1, 1
+    o.poisson.restart = 26
+    used, dc = stage()
+    fresh, dc2 = stage()
+    res = [used.initialize(o).poisson_iterations]
+    first = [dc.host(f) for f in FIELDS]
+    res.append(used.initialize(o).poisson_iterations)
+    again = [dc.host(f) for f in FIELDS]
+    res.append(fresh.initialize(o).poisson_iterations)
+    assert res[0] > 26 and res == [res[0]] * 3, res  # a restart: every vector was made
+    for n, f in enumerate(FIELDS):
+        assert np.array_equal(first[n], again[n]) and np.array_equal(first[n], dc2.host(f)), f
+    used.close()
+    fresh.close()
