@@ -3695,6 +3695,25 @@ gb_status init_solver(gb_simplec* S, const int32_t* pbc, const gb_poisson_opts& 
     return GB_OK;
 }
 
+//! However the projection ends, what its solver made beyond the stage's own
+//! arrays goes back (a solve that does not converge is the one that made every
+//! vector of its restart). The error of the projection stays the call's.
+struct InitSolverScope {
+    gb_simplec* S;
+    ~InitSolverScope()
+    {
+        gb_poisson* P = S->init_poisson;
+        if (P == nullptr) { return; }
+        if (P->borrows) {
+            P->release_chunks();
+            return;
+        }
+        cudaStreamSynchronize(S->ctx->stream);
+        delete P;
+        S->init_poisson = nullptr;
+    }
+};
+
 gb_status simplec_initialize(gb_simplec* S, const gb_state& q, const gb_init_opts& o, gb_init_result* r)
 {
     gb_ctx* ctx = S->ctx;
@@ -3787,6 +3806,7 @@ gb_status simplec_initialize(gb_simplec* S, const gb_state& q, const gb_init_opt
                                                                                      : GB_POISSON_NEUMANN);
         }
         gb_poisson_opts po = o.poisson;
+        const InitSolverScope scope{S};
         gb_status st = init_solver(S, pbc, po);
         if (st != GB_OK) { return st; }
         const bool unit = (o.alpha_h == 1 && o.alpha_v == 1);
@@ -3835,13 +3855,6 @@ gb_status simplec_initialize(gb_simplec* S, const gb_state& q, const gb_init_opt
         }
         w_from_omega(S, q.u, q.v, w.om, q.w);
         velocity_divergence(S, q.u, q.v, q.w, w.rhs);
-        // what the solve made beyond the stage's own arrays goes back
-        if (S->init_poisson->borrows) {
-            S->init_poisson->release_chunks();
-        } else {
-            gb_poisson_destroy(S->init_poisson);
-            S->init_poisson = nullptr;
-        }
     }
     dsum(S, valid_box(g, CC), w.rhs, 0, 1);
     double sums[3];

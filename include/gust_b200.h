@@ -682,7 +682,8 @@ gb_status gb_init_options_default(gb_init_opts* o);
  * z-face coefficient when alpha_v != alpha_h (u, v, Omega += the fluxes, w
  * from Omega). The projection may allocate device memory while it runs (a solver
  * where the stage's own cannot lend its arrays, vectors past those the stage
- * holds) and gives it back before the call returns. */
+ * holds) and gives it back before the call returns, whatever it returns; two
+ * arrays of split coefficients stay with the stage. */
 gb_status gb_simplec_initialize(gb_simplec* s, const gb_state* q, const gb_init_opts* o, gb_init_result* r);
 
 /* What a prolongation did (gust::ProlongResult, Source/Transfer.H:112-116). */

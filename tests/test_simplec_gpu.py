@@ -453,3 +453,45 @@ def test_gpu_initializer_with_vectors_beyond_the_stages(ctx):
         assert np.array_equal(first[n], again[n]) and np.array_equal(first[n], dc2.host(f)), f
     used.close()
     fresh.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1], ids=["borrowed arrays", "a solver of its own"])
+def test_gpu_initializer_that_fails_gives_its_memory_back(ctx, precision):
+    """A projection that does not converge within the steps of its restart
+    (every vector made: 18 volumes past the lent ones, or a whole solver's
+    for an FP32 projection on an FP64 stage) leaves the device's free memory
+    where it was, reports itself, and the next initial state has a new
+    stage's bits."""
+    import torch
+
+    import ablsteadyrans_b200 as gb
+    from ablsteadyrans_b200 import abi, workloads
+    from ablsteadyrans_b200.simplec import FIELDS, DeviceCase, SimplecStage
+
+    def stage():
+        inst = workloads.tile(96, 48, 3, precision=0)
+        inst.options.poisson.restart = 2
+        J, ax, ay, az, _ = oracle.metrics(inst.grid, inst.z)
+        dc = DeviceCase(inst.grid, inst.z, J, ax, ay, az, inst.nu, inst.gamma_theta, inst.gamma_tke, inst.q, inst.z0map)
+        return SimplecStage(ctx, dc, inst.bc, inst.physics, inst.options), dc
+
+    o = abi.InitOptions.make()
+    o.poisson.precision = precision
+    o.poisson.nu1, o.poisson.nu2, o.poisson.nu_coarse, o.poisson.restart = 0, 1, 1, 25
+    used, dc = stage()
+    used.initialize(o)
+    o.poisson.reltol, o.poisson.max_iter = 1e-14, 25
+    before = torch.cuda.mem_get_info()[0]
+    with pytest.raises(gb.GustError, match="did not converge"):
+        used.initialize(o)
+    kept = before - torch.cuda.mem_get_info()[0]
+    assert kept < 8 * dc.grid.volume, kept
+    plain = abi.InitOptions.make()
+    used.initialize(plain)
+    fresh, dc2 = stage()
+    fresh.initialize(plain)
+    for f in FIELDS:
+        assert np.array_equal(dc.host(f), dc2.host(f)), f
+    used.close()
+    fresh.close()
