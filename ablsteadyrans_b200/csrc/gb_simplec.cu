@@ -8,6 +8,7 @@
 // layer, the theta and k sweeps and the stage norms. Every reduction is
 // deterministic (block partials summed in a fixed order, maxima by bit
 // pattern), so a run repeats to the bit.
+#include "gb_branches.h"
 #include "gb_line.cuh"
 #include "gb_poisson_api.cuh"
 #include "gb_simplec.cuh"
@@ -441,12 +442,7 @@ struct gb_simplec {
     bool lin_ready{false};
     cudaStream_t capture_stream{nullptr};
     // the side streams and events of launches that do not depend on one another (Branches)
-    static constexpr int kSides = 4;
-    cudaStream_t side[kSides]{};
-    cudaEvent_t fork_ev{nullptr};
-    cudaEvent_t join_ev[kSides]{};
-    int sides{-1};   // -1: not made yet; 0: could not be made
-    bool forked{false};
+    gb::SideStreams sides;
     cudaGraphExec_t seg_exec[2]{nullptr, nullptr};
     int64_t seg_launches[2]{0, 0};
     uint64_t seg_key[2]{0, 0};
@@ -456,11 +452,6 @@ struct gb_simplec {
 
 gb_simplec::~gb_simplec()
 {
-    for (int n = 0; n < kSides; ++n) {
-        if (side[n]) { cudaStreamDestroy(side[n]); }
-        if (join_ev[n]) { cudaEventDestroy(join_ev[n]); }
-    }
-    if (fork_ev) { cudaEventDestroy(fork_ev); }
     if (poisson) { gb_poisson_destroy(poisson); }
     if (init_poisson) { gb_poisson_destroy(init_poisson); }
     for (void* p : owned) { cudaFree(p); }
@@ -498,69 +489,17 @@ float* fbuf(gb_simplec* S, int64_t n)
 
 // --------------------------------------------------- independent launches ---
 
-//! Launch sequences that do not depend on one another, each on a stream of its
-//! own between a fork and a join: on(b) sends what follows to branch b (0: the
-//! context's stream), join() makes the context's stream wait for all of them.
-//! Every side stream starts after the work queued before the fork and the
-//! context's stream goes on after the join, so callers see one stream. Under
-//! capture the branches become parallel paths of the graph. A small grid's
+//! The stage's branches (SideBranches) from the context's stream. A small grid's
 //! launches (32 x 32 x 48: five residual launches of 22 us, each on 96 of 148
 //! SMs and bound by latency) then run side by side, and a large one's fill each
 //! other's last waves. One stream while profiling, with GB_TUNE_GRAPHS = 1
 //! (every kernel alone) and inside another fork.
-class Branches {
+class Branches : public SideBranches {
 public:
-    explicit Branches(gb_simplec* S) : S_(S), main_(S->ctx->stream)
+    explicit Branches(gb_simplec* S)
+        : SideBranches(S->sides, S->ctx->stream, !S->ctx->profiling && S->ctx->tune[GB_TUNE_GRAPHS] != 1)
     {
-        if (S->forked || S->ctx->profiling || S->ctx->tune[GB_TUNE_GRAPHS] == 1 || !ready()) { return; }
-        open_ = S->forked = cudaEventRecord(S->fork_ev, main_) == cudaSuccess;
     }
-    Branches(const Branches&) = delete;
-    Branches& operator=(const Branches&) = delete;
-    ~Branches() { join(); }
-    void on(int b)
-    {
-        if (!open_) { return; }
-        if (b > 0 && !(used_ & (1u << b))) {
-            cudaStreamWaitEvent(S_->side[b - 1], S_->fork_ev, 0);
-            used_ |= 1u << b;
-        }
-        S_->ctx->stream = (b > 0) ? S_->side[b - 1] : main_;
-    }
-    //! Branch b alone: the context's stream goes on after what it was sent so far.
-    void join(int b)
-    {
-        if (!open_) { return; }
-        S_->ctx->stream = main_;
-        if (used_ & (1u << b)) {
-            cudaEventRecord(S_->join_ev[b - 1], S_->side[b - 1]);
-            cudaStreamWaitEvent(main_, S_->join_ev[b - 1], 0);
-        }
-    }
-    void join()
-    {
-        if (!open_) { return; }
-        for (int b = 1; b <= gb_simplec::kSides; ++b) { join(b); }
-        open_ = S_->forked = false;
-    }
-
-private:
-    bool ready()
-    {
-        if (S_->sides >= 0) { return S_->sides > 0; }
-        bool ok = cudaEventCreateWithFlags(&S_->fork_ev, cudaEventDisableTiming) == cudaSuccess;
-        for (int n = 0; n < gb_simplec::kSides && ok; ++n) {
-            ok = cudaStreamCreateWithFlags(&S_->side[n], cudaStreamNonBlocking) == cudaSuccess
-                 && cudaEventCreateWithFlags(&S_->join_ev[n], cudaEventDisableTiming) == cudaSuccess;
-        }
-        if (!ok) { cudaGetLastError(); }
-        S_->sides = ok ? gb_simplec::kSides : 0;
-        return ok;
-    }
-    gb_simplec* S_;
-    cudaStream_t main_;
-    unsigned used_{0};
-    bool open_{false};
 };
 
 // --------------------------------------------------------- reductions ---
