@@ -37,8 +37,8 @@ struct LineArgs {
     T* __restrict__ ebuf;
     int first;  // dold == 0: no neighbour terms, change against 0
     unsigned long long* change;  // max |dnew - dold| (nullptr: not wanted)
-    unsigned long long* clear;   // a word the sweep sets to 0 for a later one (nullptr: none)
-    const T* __restrict__ rfold;  // rhs with the lagged lateral terms folded in (the split sweep)
+    unsigned long long* clear{nullptr};   // a word the sweep sets to 0 for a later one (nullptr: none)
+    const T* __restrict__ rfold{nullptr};  // rhs with the lagged lateral terms folded in (the split sweep)
 };
 
 template <typename T, bool SMEM>
