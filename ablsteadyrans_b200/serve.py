@@ -224,28 +224,39 @@ def serve_vs_sequential(count=12, rate=2.0, seed=0, sizes=None, layers=None, max
     return serve_sweep([rate], count, seed, sizes, layers, max_iterations, budget)[0]
 
 
+def projection_bytes(inst, restart):
+    """Most bytes the initializer's projection holds for its time: it works in
+    the arrays of the stage's solver (2 `restart` + 1 vectors) and of the line
+    systems (four of seven coefficients) and makes the vectors of its own
+    restart beyond those."""
+    import ablsteadyrans_b200 as gb
+    from . import abi
+    beyond = 2 * abi.InitOptions.make().poisson.restart + 1 - (2 * restart + 1) - 4 * gb.N_COEFS
+    return 8 * inst.grid.volume * max(beyond, 0)
+
+
 def measure_peak_bytes(n, nz):
-    """Peak device bytes of one request on an n x n x nz tile: the resident
-    member plus the initializer's Poisson solver, which lives only while the
-    initial state is projected."""
+    """Peak device bytes of one request on an n x n x nz tile: what is resident
+    after the initial state and three iterations (everything made on first
+    use is there, graphs included), plus what the projection may hold."""
     import torch
 
-    import ablsteadyrans_b200 as gb
     from . import workloads
     from .batch import Member
+    from .simplec import run_drivers
     inst = workloads.tile(n, nz, 0)
     torch.cuda.synchronize()
+    torch.cuda.empty_cache()
     free0, _ = torch.cuda.mem_get_info()
     m = Member(inst)
-    opts = gb.PoissonOptions.default(precision=inst.options.precision)
-    ps = gb.PoissonSolver(m.ctx, inst.grid, m.case.z, m.case.J, [1, 1, 1, 2, 2, 1], opts)
+    m.stage.initialize()
+    run_drivers([m.native], 3, 1)
     torch.cuda.synchronize()
     free1, _ = torch.cuda.mem_get_info()
-    ps.close()
     m.close()
     del m
     torch.cuda.empty_cache()
-    return max(free0 - free1, 1), inst.grid.volume
+    return max(free0 - free1, 1) + projection_bytes(inst, inst.options.poisson.restart), inst.grid.volume
 
 
 def calibrate_footprint():

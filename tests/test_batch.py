@@ -83,6 +83,32 @@ def test_gpu_server_admits_by_footprint_and_finishes_every_request():
 
 
 @pytest.mark.gpu
+def test_gpu_footprint_model_is_what_a_request_holds():
+    """The admission's bytes of a tile between the two that the model is fitted
+    on cover what the request holds (its resident state after iterations, and
+    every vector of its projection's restart: 101 less the 17 of the stage's
+    solver and the 28 of the line systems) by no more than the admission's
+    margin of 1.1 and as much again for the fit and the allocations' rounding."""
+    import torch
+
+    from ablsteadyrans_b200 import workloads
+    from ablsteadyrans_b200.simplec import run_drivers
+    srv = serve.Server(budget=1e15, footprint=serve.calibrate_footprint())
+    inst = workloads.tile(96, 64, 1)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    m = batch.Member(inst)
+    m.stage.initialize()
+    run_drivers([m.native], 4, 1)
+    torch.cuda.synchronize()
+    held = free - torch.cuda.mem_get_info()[0] + 8 * inst.grid.volume * (101 - 17 - 28)
+    m.close()
+    need = srv.footprint(serve.Request(0, "rans", inst, 0.0))
+    assert held <= need <= 1.21 * held, (held, need)
+
+
+@pytest.mark.gpu
 def test_gpu_native_driver_equals_the_python_driver():
     """The C++ driver (gb_driver: local dtau, iteration, criterion, SER law)
     takes the same steps as the Python one: identical fields after 8 steps."""
