@@ -264,11 +264,13 @@ def bench_config(wl):
 # ------------------------------------------------- the Poisson rooflines ---
 # Algorithmic words per cell: the terrain operator apply reads phi, the
 # three a beta, J and z_nd and writes y (7); a z-line zebra relaxation of a
-# level reads phi, rhs, the three areas, J and z_nd and writes phi (8); the
-# residual of a level is an apply (7); restriction reads the fine residual
-# and writes a quarter coarse value (1.25 per fine cell), prolongation reads
-# a quarter coarse value and phi and writes phi (2.25 per fine cell).
-APPLY_WORDS, RELAX_WORDS, RESTRICT_WORDS, PROLONG_WORDS = 7, 8, 1.25, 2.25
+# level reads phi, rhs, the three areas, J and z_nd and writes phi (8), the
+# first one of a level, from a zero phi, does not read it (7); the restriction
+# of the residual reads phi, rhs, the three areas, J and z_nd and writes a
+# quarter coarse value (7.25 per fine cell: the fine residual stays in
+# registers), prolongation reads a quarter coarse value and phi and writes phi
+# (2.25 per fine cell).
+APPLY_WORDS, RELAX_WORDS, RELAX_ZERO_WORDS, RESTRICT_WORDS, PROLONG_WORDS = 7, 8, 7, 7.25, 2.25
 
 
 def mg_levels(nx, ny, max_levels, min_coarse):
@@ -289,10 +291,11 @@ def vcycle_words(nx, ny, nz, opts):
     words = 0.0
     for n, (lx, ly) in enumerate(levels):
         cells = lx * ly * nz
-        if n == len(levels) - 1:
-            words += opts.nu_coarse * RELAX_WORDS * cells
-        else:
-            words += ((opts.nu1 + opts.nu2) * RELAX_WORDS + APPLY_WORDS + RESTRICT_WORDS + PROLONG_WORDS) * cells
+        last = n == len(levels) - 1
+        down = opts.nu_coarse if last else opts.nu1  # relaxations from a zero correction
+        words += (RELAX_ZERO_WORDS + (down - 1) * RELAX_WORDS if down > 0 else 0) * cells
+        if not last:
+            words += (opts.nu2 * RELAX_WORDS + RESTRICT_WORDS + PROLONG_WORDS) * cells
     return words, len(levels)
 
 
@@ -355,8 +358,8 @@ def poisson_rooflines(ctx, wl, flush, peak, reps=12):
                 words, nlev = vcycle_words(g.nx, g.ny, g.nz, opts)
                 word = 8 if prec == 0 else 4
                 what = (f"one multigrid V-cycle ({nlev} levels, nu1 = nu2 = {opts.nu1}, {opts.nu_coarse} coarsest "
-                        f"relaxations), {'FP64' if prec == 0 else 'FP32'}; 8 words per cell and relaxation, 7 per "
-                        "residual, 1.25 restriction, 2.25 prolongation")
+                        f"relaxations), {'FP64' if prec == 0 else 'FP32'}; 8 words per cell and relaxation, 7 for a "
+                        "level's first, 7.25 residual and restriction, 2.25 prolongation")
             nbytes = words * word
             achieved = nbytes / (t / 1e3) / 1e9
             out.append({"kernel": what, "bound": "hbm", "bytes_per_launch": nbytes, "launch_ms": t,

@@ -80,7 +80,7 @@ enum {
     GB_KERNEL_LINE_SWEEP = 0,   /* z-line Thomas sweep (one launch per sweep) */
     GB_KERNEL_POISSON_APPLY,    /* terrain Poisson operator apply / residual */
     GB_KERNEL_MG_SMOOTH,        /* multigrid z-line smoother */
-    GB_KERNEL_MG_TRANSFER,      /* restriction / prolongation */
+    GB_KERNEL_MG_TRANSFER,      /* residual and restriction (one launch) / prolongation */
     GB_KERNEL_RESIDUAL,         /* control-volume residual stencils */
     GB_KERNEL_MASSFLUX,         /* mass-flux / divergence kernels */
     GB_KERNEL_COEFS,            /* implicit coefficients and row folds */

@@ -67,3 +67,16 @@ def test_single_rank_needs_no_process_group():
     import bench
     assert bench.max_over_ranks(None, 7.0, "cpu") == 7.0
     assert bench.whole_job_rate(100, 1, 4, 2.0) == pytest.approx(100 * 4 / 0.002)
+
+
+def test_vcycle_words_are_those_of_its_launches():
+    """Two levels, 4 x 4 and 2 x 2 columns of 3 cells. Fine: a relaxation from
+    zero (7), the residual with its restriction (7.25), the prolongation
+    (2.25), a relaxation (8). Coarse: one relaxation from zero and seven more."""
+    from types import SimpleNamespace
+
+    import bench
+    opts = SimpleNamespace(max_levels=12, min_coarse=2, nu1=1, nu2=1, nu_coarse=8)
+    assert bench.vcycle_words(4, 4, 3, opts) == (48 * 24.5 + 12 * 63, 2)
+    opts.nu1 = 0  # the fine correction is zero until the prolongation
+    assert bench.vcycle_words(4, 4, 3, opts) == (48 * 17.5 + 12 * 63, 2)
