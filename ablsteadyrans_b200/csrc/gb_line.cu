@@ -693,12 +693,6 @@ __device__ __forceinline__ void zline_seg_body(const LineArgs<T>& a, T* __restri
     }
 }
 
-template <typename T, bool FIRST, int L>
-__global__ void __launch_bounds__(512) zline_seg_kernel(LineArgs<T> a, T* __restrict__ inv_io, T* __restrict__ cp_io)
-{
-    zline_seg_body<T, FIRST, L>(a, inv_io, cp_io, blockIdx.x);
-}
-
 //! The split sweep's first half: the right-hand side with the lagged lateral
 //! terms, r' = rhs + a_XM d_XM + a_XP d_XP + a_YM d_YM + a_YP d_YP (the
 //! segmented sweep's fold, in its operation order), one thread per point,
@@ -855,9 +849,6 @@ gb_status zline_sweeps(gb_ctx* ctx, const gb_grid& g, int loc, const T* A, const
 {
     const int ni = ext_x(g, loc), nj = ext_y(g, loc), nk = ext_z(g, loc);
     const int64_t vol = volume(g);
-    // Ping-pong: sweep s writes buf[(sweeps - 1 - s) & 1], so the last sweep lands in delta.
-    T* tmp = static_cast<T*>(scratch(ctx, kSlotLineNext, sizeof(T) * vol));
-    if (tmp == nullptr) { return GB_OOM; }
     const size_t smem = line_smem_bytes<T>(nk);
     const int segL = seg_levels(ctx);
     const int segW = seg_warps(nk, segL);
@@ -881,6 +872,9 @@ gb_status zline_sweeps(gb_ctx* ctx, const gb_grid& g, int loc, const T* A, const
         unsigned long long* words[1] = {change_word};
         return zline_sweeps_multi<T>(ctx, g, 1, locs, As, aps, rhss, sweeps, deltas, words);
     }
+    // Ping-pong: sweep s writes buf[(sweeps - 1 - s) & 1], so the last sweep lands in delta.
+    T* tmp = static_cast<T*>(scratch(ctx, kSlotLineNext, sizeof(T) * vol));
+    if (tmp == nullptr) { return GB_OOM; }
     const bool factored = (scratch_kind == LineScratch::factored);
     const bool pipelined = factored || (scratch_kind == LineScratch::pipelined);
     T* inv = nullptr;

@@ -2962,7 +2962,6 @@ gb_status scalar_sweeps(gb_simplec* S, const gb_state& q, const double* dtau, bo
     gb_ctx* ctx = S->ctx;
     const gb_grid g = S->g;
     SimplecWork& w = S->w;
-    const int64_t cs = volume(g);
     const int eqs[2] = {F_THETA, F_TKE};
     double* fields[2] = {q.theta, q.tke};
     const double* Rq[2] = {w.R[4], w.R[5]};
