@@ -528,8 +528,8 @@ __device__ __forceinline__ void line_factor_column(const gb_grid& g, T* __restri
     }
 }
 
-//! Every level's line tridiagonal (k_line_tridiag) in one launch and every
-//! level's column factorisation (k_line_factor) in another: the levels are
+//! Every level's line tridiagonal (line_tridiag) in one launch and every
+//! level's column factorisation (line_factor_column) in another: the levels are
 //! independent, and one launch over all of them replaces two per level (the
 //! coarse levels' launches were latency for a few hundred cells).
 template <typename T>
@@ -584,7 +584,7 @@ __global__ void k_line_factor_all(const __grid_constant__ LineLevels<T> L)
 }
 
 //! Zebra relaxation, second half: on every column of the colour x += T^{-1} r
-//! with the factors of k_line_factor (e_k = (r_k - D_k e_{k-1}) / m_k, then
+//! with the factors of line_factor_column (e_k = (r_k - D_k e_{k-1}) / m_k, then
 //! x_k = e_k - c'_k x_{k+1}), the column's r, D, 1/m, c' staged R levels ahead
 //! into shared memory with asynchronous copies (c', e' kept in shared memory).
 //! Used when a whole column does not fit the staged kernel below.
@@ -763,7 +763,7 @@ __global__ void __launch_bounds__(256) k_color_relax_fused(gb_grid g, PBC b, int
 
 //! Zebra relaxation, second half, with the column's levels split among the
 //! warps of a block: x += T^{-1} r on every column of the colour with the
-//! factors of k_line_factor (e_k = (r_k - D_k e_{k-1}) / m_k, then x_k = e_k
+//! factors of line_factor_column (e_k = (r_k - D_k e_{k-1}) / m_k, then x_k = e_k
 //! - c'_k x_{k+1}). A block holds 32 columns of the colour along one row and
 //! ceil(nz / L) warps; each thread loads its L levels' r, D, 1/m, c' and x at
 //! once (in-range clamped indices: no load behind a branch), runs the

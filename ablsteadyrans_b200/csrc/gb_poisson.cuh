@@ -336,7 +336,9 @@ __device__ __forceinline__ void line_tridiag(const gb_grid& g, const PBC& b, con
     if (!b.per_y && j == 0 && b.syl < 0) { cyl = T(2) * dyinv; }
     if (!b.per_y && j == g.ny - 1 && b.syh < 0) { cyh = T(2) * dyinv; }
     c -= (myh * AY[at(g, i, j + 1, k)] * cyh + myl * AY[at(g, i, j, k)] * cyl) * dyinv;
-    // 1 / h_zeta of the two z-faces: the mesh ratios (the same quotients, taken once per mesh)
+    // 1 / h_zeta of the two z-faces: the mesh ratios, taken once per mesh. In FP64
+    // the same quotients; the FP32 hierarchy's are FP64's rounded once, where
+    // differences of heights rounded to FP32 used to be divided
     const T hzi_hi = hz[at(g, i, j, k + 1)], hzi_lo = hz[at(g, i, j, k)];
     const T mzl = (k != 0) ? T(1) : T(0);
     const T mzh = ((b.zf & TP_ZHI) && k == g.nz - 1) ? T(0) : T(1);

@@ -904,8 +904,8 @@ void velocity_divergence(gb_simplec* S, const double* u, const double* v, const 
     const double* az = S->mesh.az;
     const double* J = S->mesh.detJ;
     // a thread takes L levels of a column: each z-face's Omega is evaluated once
-    // and serves the cells below and above it. Four levels where they leave eight
-    // blocks an SM (128 x 128 x 64: 24 us, 29 with a cell a thread), else a cell a
+    // and serves the cells below and above it. Four levels where they leave six
+    // 256-thread blocks an SM (128 x 128 x 64: 24 us, 29 with a cell a thread), else a cell a
     // thread (32 x 32 x 48: 7.5 us, 13 with four levels, 12 blocks)
     auto launch = [&](auto Lc) {
         constexpr int L = decltype(Lc)::value;
@@ -1418,7 +1418,7 @@ __device__ __forceinline__ void fused_face(const FusedResidualArgs& a, int i, in
 //! The faces past a block's last column: the first warp evaluates them for the
 //! eight rows of kEdgeLevels levels at once, a lane a face. With the last lane of
 //! each row's warp evaluating its own, every warp went through the x face twice
-//! a level (a level: 5.6 face evaluations a warp, now 4.3 at two levels a block).
+//! a level (a level: 4.6 face evaluations a warp, now 3.7 at two levels a block).
 constexpr int kEdgeLevels = 4;
 static_assert(kEdgeLevels * kFusedTy == kFusedTx, "a lane a face");
 
@@ -2907,7 +2907,9 @@ uint64_t segment_key(const gb_simplec* S, const gb_state& q, const double* dtau)
 //! iteration (it sizes the scratch and sets the kernels' attributes), while
 //! profiling and with GB_TUNE_GRAPHS = 1; else the graph, captured on the
 //! stage's stream when its key changed, launched on the context's stream.
-//! The kernels and their order are the same either way.
+//! The kernels are the same either way and each comes after those it depends
+//! on; launches of different branches have no order in a graph, while profiling
+//! and GB_TUNE_GRAPHS = 1 put them on one stream (Branches).
 template <typename F>
 gb_status run_segment(gb_simplec* S, int id, uint64_t key, F&& body)
 {

@@ -121,13 +121,16 @@ enum {
                                    0 auto (= 1), 1 shared memory, 2 the global arrays (c' stored, e' in the
                                    output array), 3 e' in shared memory and c' read again from its stored
                                    array (L2): less shared memory per warp, more warps per SM */
-    GB_TUNE_MG_FUSED_RELAX,     /* one launch per colour of the zebra line relaxation: 0 auto (= 1), 1 never
-                                   (the residual and the solve as two launches), 2 the residual in shared memory
+    GB_TUNE_MG_FUSED_RELAX,     /* one launch per colour of the zebra line relaxation: 0 auto (= 1), 1 on the
+                                   levels that then need at most one block an SM (a cell a thread; the
+                                   residual and the solve as two launches on the others), 2 the residual in shared memory
                                    and one thread per column's solve, on every level, 3 that on the levels of at
                                    most 1024 columns, 4 segmented (the column's levels split among the warps of
                                    a block, the residual in registers; columns of more than 128 levels: 1) */
     GB_TUNE_GRAPHS,             /* CUDA graphs for launch sequences without a host synchronisation (the
-                                   multigrid V-cycle): 0 default (on), 1 off (every kernel launched alone) */
+                                   multigrid V-cycle, the stage's iteration) and the stage's side streams for
+                                   launches that do not depend on one another: 0 default (on), 1 off (every
+                                   kernel launched alone, on the context's stream) */
     GB_TUNE_MG_SOLVE,           /* the column solves of the two-launch zebra relaxation: 0 default (the
                                    column's levels split among the warps of a block), 1 one thread per column */
     GB_TUNE_LINE_FIRST,         /* the first sweep of a segmented solve (the column factorisation): 0 default
@@ -137,7 +140,8 @@ enum {
                                    segmented zebra relaxation (default 4, 8 for columns of more than 64
                                    levels): 0 default, 4 or 8 */
     GB_TUNE_RESIDUAL,           /* the SIMPLEC residual's convection, diffusion and pressure gradient and
-                                   the implicit coefficients: 0 default (one launch per equation, each
+                                   the implicit coefficients (without a damping layer their rows and
+                                   systems in the same launch, but for 1): 0 default (one launch per equation, each
                                    face evaluated once per block, 2 levels per block), 1 one thread per
                                    point (the residual's fluxes and divergences as separate launches),
                                    N >= 2 the per-equation launch with N levels per block */
